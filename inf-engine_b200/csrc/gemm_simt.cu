@@ -6,7 +6,13 @@
 // Every output element is one accumulator that walks k = 0..K-1 in ascending
 // order, so a row's result does not depend on how many rows share the launch.
 // A, W and C may each be float32 or bfloat16; products and sums are float32.
+//
+// A product of all float32 whose rows lie on 16 bytes goes to gemm_f32.cu, which reads W once at HBM speed for a few rows and
+// keeps the multipliers busy for many; this kernel keeps mixed types and rows off that alignment.
 #include "common.cuh"
+
+int gemm_f32_takes(const void* A, const void* W, int K, int lda, int ldw);
+int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream);
 
 #define GS_BM 64
 #define GS_BN 64
@@ -85,7 +91,10 @@ extern "C" int ie_gemm_simt(const void* A, int a_dtype, const void* W, int w_dty
   if (K <= 0) return IE_BAD_SIZE;
   const int code = a_dtype * 4 + w_dtype * 2 + c_dtype;
   switch (code) {
-    case 0: return launch_gemm<float, float, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    case 0:
+      if (gemm_f32_takes(A, W, K, lda, ldw))
+        return gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc, stream);
+      return launch_gemm<float, float, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     case 2: return launch_gemm<float, bf16, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     case 4: return launch_gemm<bf16, float, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     case 5: return launch_gemm<bf16, float, bf16>(A, W, C, M, N, K, lda, ldw, ldc, stream);

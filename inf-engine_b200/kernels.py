@@ -1265,23 +1265,33 @@ def gated_delta_library(head_dim: int, v_head_dim: int):
         defines = {"IE_GD_DK": key[0], "IE_GD_DV": key[1], **BUILD_DEFINES.get("gated_delta", {})}
         lib = load_library(f"gated_delta_k{key[0]}_v{key[1]}", ["gated_delta.cu"], defines)
         P, I, F = c_void_p, c_int, c_float
-        lib.ie_gated_delta.argtypes = [P, P, P, I, I, P, P, I, P, I, P, P, P, I, P, P, I, P, P, I, I, I, I, I, F, F, I, I, P]
+        lib.ie_gated_delta.argtypes = [P, P, P, I, I, P, P, I, P, I, P, P, P, I, P, P, I, P, P, I, I, I, I, I, F, F, I, I, P, I, I, P]
         lib.ie_gated_delta.restype = c_int
+        lib.ie_gated_delta_scratch_floats.argtypes = [I, I, I]
+        lib.ie_gated_delta_scratch_floats.restype = c_longlong
         _gated_delta[key] = lib
         _apply_check_limits()
     return lib
 
 
+def gated_delta_scratch_floats(n_tokens: int, n_requests: int, n_heads: int, head_dim: int, v_head_dim: int) -> int:
+    """Floats of scratch that the chunked form of ``gated_delta`` wants; 0: these head sizes have no such form."""
+    return int(gated_delta_library(head_dim, v_head_dim).ie_gated_delta_scratch_floats(n_tokens, n_requests, n_heads))
+
+
 def gated_delta(q, k, v, b_pre, a_pre, gate, a_log, dt_bias, out_gain, state, out, q_start, slots, n_requests: int,
                 n_heads: int, n_kv_heads: int, head_dim: int, v_head_dim: int, key_eps: float, norm_eps: float,
-                write_state: bool = True) -> None:
+                write_state: bool = True, scratch: torch.Tensor | None = None, max_q_len: int = 0) -> None:
     """One step of the gated delta rule for every (request, head) of the batch.
 
     ``q, k`` [n, kv_heads * head_dim] and ``v`` [n, heads * v_head_dim] (after their convolutions and SiLU), ``b_pre,
     a_pre`` [n, heads], ``gate`` [n, heads * v_head_dim]: row-strided views in the activation type; ``a_log, dt_bias``
     [heads] and ``out_gain`` [v_head_dim] of one type; ``state`` float32 [slots, heads, head_dim, v_head_dim], read and
     (with ``write_state``) written at ``slots[request]``; ``out`` [n, heads * v_head_dim] in the activation type: the
-    normed, gated result for the output projection."""
+    normed, gated result for the output projection.  With ``scratch`` (float32, ``gated_delta_scratch_floats``) the tokens
+    are taken in chunks, the longest request's being ``max_q_len``; without it one after another."""
+    assert scratch is None or (scratch.dtype is torch.float32 and scratch.is_contiguous() and max_q_len > 0 and scratch.numel()
+                               >= gated_delta_scratch_floats(q.shape[0], n_requests, n_heads, head_dim, v_head_dim) > 0)
     for t in (q, k, v, b_pre, a_pre, gate, out):
         assert t.dtype == q.dtype and t.stride(1) == 1
     assert q.stride(0) == k.stride(0) and b_pre.stride(0) == a_pre.stride(0)
@@ -1292,7 +1302,7 @@ def gated_delta(q, k, v, b_pre, a_pre, gate, a_log, dt_bias, out_gain, state, ou
         _ptr(q), _ptr(k), _ptr(v), q.stride(0), v.stride(0), _ptr(b_pre), _ptr(a_pre), b_pre.stride(0), _ptr(gate),
         gate.stride(0), _ptr(a_log), _ptr(dt_bias), _ptr(out_gain), dtype_code(a_log.dtype), _ptr(state), _ptr(out),
         out.stride(0), _ptr(q_start), _ptr(slots), n_requests, n_heads, n_kv_heads, head_dim, v_head_dim, float(key_eps),
-        float(norm_eps), 1 if write_state else 0, dtype_code(q.dtype), _stream()),
+        float(norm_eps), 1 if write_state else 0, dtype_code(q.dtype), _ptr(scratch), int(max_q_len), q.shape[0], _stream()),
         f"gated_delta(head_dim={head_dim}, v_head_dim={v_head_dim}, heads={n_heads}/{n_kv_heads})")
 
 

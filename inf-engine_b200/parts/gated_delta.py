@@ -28,6 +28,10 @@ from .linear import Linear
 from .registry import register_mixer
 
 
+CHUNK_MIN_TOKENS = 64                # longest request of a step from which chunks beat a token after another
+CHUNK_MAX_SCRATCH = 1 << 28          # floats (1 GB; 20,000 tokens of 32 heads of 64 x 64): longer steps go token after token
+
+
 def conv_state_requirement(taps: int, channels: int, dtype: torch.dtype) -> CacheRequirement:
     """The state of a short convolution: a sequence's last ``taps - 1`` inputs, oldest first."""
     return CacheRequirement(kind="state", state_shape=(max(taps - 1, 0), channels), state_dtype=dtype)
@@ -105,8 +109,13 @@ class GatedDeltaMixer:
         b_pre = proj[:, c0 + self.vw:c0 + self.vw + s.n_heads]
         a_pre = proj[:, c0 + self.vw + s.n_heads:]
         mixed = rt.ws.take("gated_delta_mixed", (n, self.vw), rt.act_dtype)
+        scratch = None
+        if ctx.max_q_len >= CHUNK_MIN_TOKENS:
+            floats = kernels.gated_delta_scratch_floats(n, ctx.n_requests, s.n_heads, s.head_dim, s.v_head_dim)
+            if 0 < floats <= CHUNK_MAX_SCRATCH:
+                scratch = rt.ws.take("gated_delta_chunks", (floats,), torch.float32)
         kernels.gated_delta(conv[:, :self.qk], conv[:, self.qk:2 * self.qk], conv[:, 2 * self.qk:], b_pre, a_pre, gate,
                             self.a_log, self.dt_bias, self.out_gain, state.state, mixed, ctx.q_start, ctx.slots,
                             ctx.n_requests, s.n_heads, s.n_kv_heads, s.head_dim, s.v_head_dim, s.key_eps, s.norm_eps,
-                            write_state=cache.write)
+                            write_state=cache.write, scratch=scratch, max_q_len=ctx.max_q_len)
         return self.o(mixed, rt.ws.take("mixer_out", (n, s.hidden), rt.act_dtype))

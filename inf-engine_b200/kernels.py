@@ -81,6 +81,8 @@ def core():
         lib.ie_rope_kv_write.argtypes = [P, P, P, I, I, P, P, P, P, P, P, I, I, I, I, I, I, I, P]
         lib.ie_silu_mul.argtypes = [P, P, I, I, I, I, I, P]
         lib.ie_attention_general.argtypes = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, P, I, I, F, I, I, I, P, F, P, I, P]
+        lib.ie_attention_ordered_rows.argtypes = [P] * 7 + [I] * 11 + [F, I, P, I, P, I, P]
+        lib.ie_attention_ordered_rows.restype = c_int
         lib.ie_layernorm.argtypes = [P, P, P, P, I, P, I, P, I, I, F, P]
         lib.ie_embed_bigram.argtypes = [P, P, P, P, I, P, P, I, P, P, I, I, I, I, L, L, P]
         lib.ie_add_bias.argtypes = [P, I, P, I, I, I, I, P]
@@ -358,6 +360,24 @@ def attention_rows(q: torch.Tensor, out: torch.Tensor, kpool: torch.Tensor, vpoo
 
 
 # -------------------------------------------------------------------------- gemm
+def attention_ordered_rows(q: torch.Tensor, out: torch.Tensor, kpool: torch.Tensor, vpool: torch.Tensor, block_table: torch.Tensor,
+                           q_start: torch.Tensor, ctx_before: torch.Tensor, n_requests: int, max_rows: int, n_heads: int,
+                           n_kv_heads: int, head_dim: int, page_size: int, window: int | None, scale: float,
+                           score_bias: torch.Tensor | None = None, head_scale: torch.Tensor | None = None,
+                           v_head_dim: int | None = None) -> None:
+    """``attention_general`` for the requests that bring at most ``max_rows`` (token, head-in-group) rows, a block per (token,
+    query head), with the same bits; the others are left alone.  No kept first keys, chunks, sink, cap or gate."""
+    assert q.stride(1) == 1 and out.stride(1) == 1 and kpool.dtype == vpool.dtype == q.dtype == out.dtype
+    assert block_table.dtype == torch.int32 and block_table.stride(1) == 1
+    _score_extras(score_bias, head_scale, n_heads)
+    _check(core().ie_attention_ordered_rows(
+        _ptr(q), _ptr(out), _ptr(kpool), _ptr(vpool), _ptr(block_table), _ptr(q_start), _ptr(ctx_before), q.stride(0),
+        out.stride(0), block_table.stride(0), q.shape[0], n_requests, max_rows, n_heads, n_kv_heads, head_dim, page_size,
+        int(window or 0), float(scale), dtype_code(q.dtype), _ptr(score_bias),
+        score_bias.shape[1] if score_bias is not None else 0, _ptr(head_scale), int(v_head_dim or head_dim), _stream()),
+        f"attention_ordered_rows(head_dim={head_dim}, heads={n_heads}/{n_kv_heads})")
+
+
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     """out[M,N] = a[M,K] @ w[N,K]^T in float32 arithmetic."""
     m, k = a.shape

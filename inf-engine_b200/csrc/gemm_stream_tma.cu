@@ -593,6 +593,188 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 2 : 1) gemm_stream_tma_kern
 #endif
 }
 
+// ---------------------------------------------------------------- the experts of a few tokens
+// The (token, choice) pairs lie sorted by expert and `tiles` names (expert, first position, rows <= 16) of every expert that
+// some token chose: the product is a read of those experts' weights.  Units of 8 NT weight rows run over all tiles, block
+// after block, through the same ring; which experts there are is known only when the kernel ahead has finished, so nothing
+// is fetched before.  Against blocks that each load 8 rows for themselves and then leave (routed.cu): 16 experts of
+// 4,096 x 2,048 for 8 tokens, two each: MOE_RING_MEASURED.
+struct GroupedParams {
+  const bf16* A;
+  const bf16* W;            // [experts, N, K]
+  void* C;
+  const int* sorted;        // pair at every sorted position
+  const int* tiles;         // [max_tiles, 4]; the number of tiles in word 3 of the first
+  int max_tiles, N, K, lda, ldc, top, gather, scatter;
+  int ks, n_stages;
+  float act_alpha, act_limit, act_offset, act_cubic;
+};
+
+template <int NT, int EPI>
+__global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
+  constexpr int UNIT_ROWS = 8 * NT;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) unsigned long long bars[2 * MAX_STAGES];   // full[], empty[]
+  __shared__ float red[2][CONSUMER_WARPS][4 * NT][32];
+  __shared__ volatile int failed;
+  pdl_trigger();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t w_pitch = (uint32_t)p.ks * 2 + ROW_PAD, slot_bytes = UNIT_ROWS * w_pitch, ring = smem_addr(smem);
+  const uint32_t full0 = smem_addr(&bars[0]), empty0 = smem_addr(&bars[MAX_STAGES]);
+  if (tid == 0) {
+    failed = 0;
+    for (int s = 0; s < p.n_stages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, CONSUMER_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  pdl_wait();
+  const int n_tiles = max(0, min(p.tiles[3], p.max_tiles));
+  const int per_tile = (p.N + UNIT_ROWS - 1) / UNIT_ROWS, n_units = n_tiles * per_tile;
+  const int k_stages = p.K / p.ks;
+  int s = 0;
+  uint32_t phase = 0;
+  if (warp == CONSUMER_WARPS) {
+    // producer: lane r copies weight row r of the unit
+    bool ok = true;
+    const uint32_t row_bytes = (uint32_t)p.ks * 2;
+    const uint64_t pol = l2_evict_first_policy();
+    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+      const int tile = u / per_tile, n0 = (u - tile * per_tile) * UNIT_ROWS, rows = min(UNIT_ROWS, p.N - n0);
+      const bf16* src = p.W + ((size_t)p.tiles[4 * tile] * p.N + n0 + (lane < rows ? lane : 0)) * p.K;
+      for (int ksi = 0; ksi < k_stages; ++ksi) {
+        const uint32_t bar = full0 + 8 * s;
+        if (lane == 0) {
+          ok = mbar_wait(empty0 + 8 * s, phase ^ 1);
+          if (ok) mbar_expect_tx(bar, row_bytes * rows);
+        }
+        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        if (!ok) break;
+        if (lane < rows) bulk_copy(ring + s * slot_bytes + lane * w_pitch, src + (size_t)ksi * p.ks, row_bytes, bar, pol);
+        if (++s == p.n_stages) { s = 0; phase ^= 1; }
+      }
+    }
+    if (!ok && lane == 0) {
+      atomicExch(&g_stream_error, 1);
+      failed = 1;
+      for (int i = 0; i < 4096; ++i) __nanosleep(64);   // copies already issued land in this block's shared memory
+    }
+    return;
+  }
+  if (warp == CONSUMER_WARPS + 1) {
+    const int gg = lane >> 2, tt = lane & 3;
+    int parity = 0;
+    for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+      const int tile = u / per_tile, n0 = (u - tile * per_tile) * UNIT_ROWS;
+      const int pos0 = p.tiles[4 * tile + 1], rows = p.tiles[4 * tile + 2];
+      int at[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) at[h] = gg + 8 * h < rows ? (p.scatter ? p.sorted[pos0 + gg + 8 * h] : pos0 + gg + 8 * h) : -1;
+      named_sync(2 + parity);                                // every consumer warp has left its sums
+      if (!failed) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int n = n0 + nt * 8 + tt * 2;
+            float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+            for (int w = 0; w < CONSUMER_WARPS; ++w) {
+              v0 += red[parity][w][nt * 4 + h * 2][lane];
+              v1 += red[parity][w][nt * 4 + h * 2 + 1][lane];
+            }
+            if (at[h] >= 0 && n < p.N) {
+              const bool has1 = n + 1 < p.N;
+              if (EPI == EPI_GLU) {
+                ((bf16*)p.C)[(size_t)at[h] * p.ldc + (n >> 1)] = __float2bfloat16_rn(stream_glu(p, v0, v1));
+              } else if (EPI == EPI_RELU2) {
+                bf16* c = (bf16*)p.C + (size_t)at[h] * p.ldc + n;
+                c[0] = __float2bfloat16_rn(stream_relu2(v0));
+                if (has1) c[1] = __float2bfloat16_rn(stream_relu2(v1));
+              } else {
+                float* c = (float*)p.C + (size_t)at[h] * p.ldc + n;
+                c[0] = v0;
+                if (has1) c[1] = v1;
+              }
+            }
+          }
+        }
+      }
+      if (u + 2 * (int)gridDim.x < n_units) named_arrive(4 + parity);   // the consumers may write this buffer again
+      parity ^= 1;
+    }
+    return;
+  }
+  // consumers: a warp takes an eighth of every stage's k
+  const int g = lane >> 2, t = lane & 3;
+  const int kw = warp * (p.ks / CONSUMER_WARPS), chunks = p.ks / (CONSUMER_WARPS * 32);
+  int parity = 0, n_done = 0, tile_now = -1;
+  const bf16 *xa = p.A, *xb = p.A;
+  bool va = false, vb = false, dead = false;
+  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+    const int tile = u / per_tile;
+    if (tile != tile_now) {
+      tile_now = tile;
+      const int pos0 = p.tiles[4 * tile + 1], rows = p.tiles[4 * tile + 2];
+      va = g < rows;
+      vb = g + 8 < rows;
+      const int ra = !va ? 0 : (p.gather ? p.sorted[pos0 + g] / p.top : pos0 + g);
+      const int rb = !vb ? 0 : (p.gather ? p.sorted[pos0 + g + 8] / p.top : pos0 + g + 8);
+      xa = p.A + (size_t)ra * p.lda + kw + t * 8;
+      xb = p.A + (size_t)rb * p.lda + kw + t * 8;
+    }
+    float acc[NT][2][4] = {};
+    for (int ksi = 0; ksi < k_stages; ++ksi) {
+      // the activations come from L2 and do not depend on the stage: asked for before the wait
+      uint4 x0[8], x1[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        x0[c] = (va && c < chunks) ? __ldcg(reinterpret_cast<const uint4*>(xa + ksi * p.ks + c * 32)) : make_uint4(0u, 0u, 0u, 0u);
+        x1[c] = (vb && c < chunks) ? __ldcg(reinterpret_cast<const uint4*>(xb + ksi * p.ks + c * 32)) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      if (!dead && (failed || !mbar_wait(full0 + 8 * s, phase))) {
+        dead = true;
+        if (lane == 0) { atomicExch(&g_stream_error, 2); failed = 1; }
+      }
+      if (!dead) {
+        const uint32_t wbase = ring + s * slot_bytes + g * w_pitch + (kw + t * 8) * 2;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          if (c < chunks) {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+              const uint4 w = lds128(wbase + nt * 8 * w_pitch + c * 64);
+              mma16816(acc[nt][0], x0[c].x, x1[c].x, x0[c].y, x1[c].y, w.x, w.y);
+              mma16816(acc[nt][1], x0[c].z, x1[c].z, x0[c].w, x1[c].w, w.z, w.w);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8 * s);
+        if (++s == p.n_stages) { s = 0; phase ^= 1; }
+      }
+    }
+    if (n_done >= 2) named_sync(4 + parity);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) red[parity][warp][nt * 4 + e][lane] = acc[nt][0][e] + acc[nt][1][e];
+    named_arrive(2 + parity);
+    parity ^= 1;
+    ++n_done;
+  }
+}
+
+template <int NT, int EPI>
+int launch_ring(const GroupedParams& p, int n_sms, size_t smem, cudaStream_t stream) {
+  static const cudaError_t ready =
+      cudaFuncSetAttribute(moe_ring_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024);
+  if (ready != cudaSuccess) return (int)ready;
+  return launch_k(moe_ring_kernel<NT, EPI>, n_sms, THREADS, smem, stream, p);
+}
+
 template <int NT, int PRO, int EPI, bool XS>
 int launch_xs(const TmaParams& p, int n_sms, size_t smem, cudaStream_t stream) {
   static bool attr = false;
@@ -742,5 +924,32 @@ extern "C" int ie_gemm_stream_tma(const void* A, const void* W, void* C, const v
     if (epi == EPI_GLU) return launch_tma<PRO_PLAIN, EPI_GLU>(p, nt, n_sms, smem, stream);
     return IE_BAD_DTYPE;
   }
+  return IE_BAD_DTYPE;
+}
+
+// The experts' product of at most 16 tokens: tiles of at most 16 rows.  epi 1 float32 store, 5 square of relu, 6 gated activation.
+extern "C" int ie_moe_ring(const void* A, const void* W, void* C, const int* sorted, const int* tiles, int max_tiles, int N, int K,
+                           int lda, int ldc, int top, int gather, int scatter, int epi, int n_sms, float act_alpha, float act_limit,
+                           float act_offset, float act_cubic, cudaStream_t stream) {
+  if (N <= 0 || max_tiles <= 0) return IE_OK;
+  if (K <= 0 || K % 256 || (lda & 7) || n_sms <= 0 || top <= 0 || (long long)max_tiles * ((N + 7) / 8) > 0x7fffffffLL) return IE_BAD_SIZE;
+  if (((uintptr_t)A | (uintptr_t)W) & 15) return IE_BAD_ALIGN;
+  if (epi == EPI_GLU && (N & 1)) return IE_BAD_SIZE;
+  GroupedParams p;
+  p.A = (const bf16*)A; p.W = (const bf16*)W; p.C = C; p.sorted = sorted; p.tiles = tiles; p.max_tiles = max_tiles;
+  p.N = N; p.K = K; p.lda = lda; p.ldc = ldc; p.top = top; p.gather = gather; p.scatter = scatter;
+  p.act_alpha = act_alpha; p.act_limit = act_limit; p.act_offset = act_offset; p.act_cubic = act_cubic;
+  // units of 16 rows halve the reads of the activations; 8 rows where 16 would leave an expert fewer units than SMs
+  const int nt = N >= 16 * n_sms ? 2 : 1;
+  p.ks = K % 1024 == 0 ? 1024 : (K % 512 == 0 ? 512 : 256);
+  const size_t stage = (size_t)8 * nt * ((size_t)p.ks * 2 + ROW_PAD);
+  p.n_stages = (int)(190 * 1024 / stage);
+  if (p.n_stages > MAX_STAGES) p.n_stages = MAX_STAGES;
+  const size_t smem = p.n_stages * stage;
+#define RING_GO(EPI) return nt == 2 ? launch_ring<2, EPI>(p, n_sms, smem, stream) : launch_ring<1, EPI>(p, n_sms, smem, stream)
+  if (epi == EPI_F32) RING_GO(EPI_F32);
+  if (epi == EPI_RELU2) RING_GO(EPI_RELU2);
+  if (epi == EPI_GLU) RING_GO(EPI_GLU);
+#undef RING_GO
   return IE_BAD_DTYPE;
 }

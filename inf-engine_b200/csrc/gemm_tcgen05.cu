@@ -55,6 +55,8 @@ struct TcParams {
   const int* tiles;
   const int* place;
   int max_tiles;
+  // block-diagonal form: output columns in groups of diag_n, group b reads columns b K .. of A (0: every column reads all of A)
+  int diag_n;
 };
 
 // the gated activation of the SILU_MUL epilogue: silu(g) * u, or with the options above
@@ -323,12 +325,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
         const int mt = t % m_tiles, n0 = (t / m_tiles) * BN;
         const int m0 = GROUPED ? p.tiles[4 * mt + 1] : mt * BM;
         const int w0 = GROUPED ? p.tiles[4 * mt] * p.N + n0 : n0;      // the expert's own rows of the stacked weights
+        const int a_k0 = (!GROUPED && p.diag_n) ? (n0 / p.diag_n) * p.K : 0;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (failed || !tc_mbar_wait(empty0 + 8 * s, phase ^ 1)) { atomicExch(&g_tc_error, 1); failed = 1; break; }
           const uint32_t bar = full0 + 8 * s;
           tc_mbar_expect_tx(bar, STAGE_BYTES);
           const uint32_t a_dst = ring + s * STAGE_BYTES, w_dst = a_dst + A_BYTES;
-          tma_load_2d(a_dst, &map_a, kb * BK, m0, bar);
+          tma_load_2d(a_dst, &map_a, a_k0 + kb * BK, m0, bar);
           tma_load_2d(w_dst, &map_w, kb * BK, w0, bar);
           if (++s == p.n_stages) { s = 0; phase ^= 1; }
         }
@@ -508,7 +511,7 @@ extern "C" int ie_gemm_tcgen05_act(const void* A, const void* W, void* C, int M,
   p.act_general = act_general; p.act_alpha = act_alpha; p.act_limit = act_limit; p.up_offset = up_offset;
   p.act_cubic = act_cubic;
   p.staged = (((uintptr_t)C & 15) == 0 && ((size_t)ldc * (epi == TC_EPI_RESIDUAL ? 4 : 2)) % 16 == 0) ? 1 : 0;
-  p.tiles = nullptr; p.place = nullptr; p.max_tiles = 0;
+  p.tiles = nullptr; p.place = nullptr; p.max_tiles = 0; p.diag_n = 0;
   return bn == 256 ? launch_tc<256, false>(ma, mw, p, n_sms, stream) : launch_tc<128, false>(ma, mw, p, n_sms, stream);
 }
 
@@ -536,9 +539,30 @@ extern "C" int ie_gemm_tcgen05_grouped(const void* A, const void* W, void* C, co
   TcParams p;
   p.C = C; p.M = n_rows; p.N = N; p.K = K; p.ldc = ldc; p.epi = epi; p.n_stages = 0;
   p.act_general = 1; p.act_alpha = act_alpha; p.act_limit = act_limit; p.up_offset = up_offset; p.act_cubic = act_cubic;
-  p.tiles = tiles; p.place = place; p.max_tiles = max_tiles;
+  p.tiles = tiles; p.place = place; p.max_tiles = max_tiles; p.diag_n = 0;
   p.staged = (((uintptr_t)C & 15) == 0 && ((size_t)ldc * (epi == TC_EPI_F32 ? 4 : 2)) % 16 == 0) ? 1 : 0;
   return bn == 256 ? launch_tc<256, true>(ma, mw, p, n_sms, stream) : launch_tc<128, true>(ma, mw, p, n_sms, stream);
+}
+
+// A block-diagonal matrix applied to rows, float32 result: W [blocks, n, K], block b maps columns b K .. of A to columns b n ..
+// of C.  n must hold whole tiles (a multiple of 128).
+extern "C" int ie_gemm_tcgen05_diag(const void* A, const void* W, float* C, int M, int blocks, int n, int K, int lda, int ldc,
+                                    int n_sms, cudaStream_t stream) {
+  if (n_sms <= 0 || blocks <= 0 || n % 128) return IE_BAD_SIZE;
+  if (M <= 0) return IE_OK;
+  if ((long long)blocks * n > 0x7fffffffLL || (long long)blocks * K > 0x7fffffffLL) return IE_BAD_SIZE;
+  if (!ie_gemm_tcgen05_supports(M, n, K, lda, K)) return IE_BAD_SIZE;
+  if (((uintptr_t)A | (uintptr_t)W) & 15) return IE_BAD_ALIGN;
+  const int bn = n % 256 == 0 ? 256 : 128;
+  CUtensorMap ma, mw;
+  int rc = make_map(&ma, A, M, blocks * K, lda, BM);
+  if (rc) return rc;
+  rc = make_map(&mw, W, blocks * n, K, K, bn);
+  if (rc) return rc;
+  TcParams p = {};
+  p.C = C; p.M = M; p.N = blocks * n; p.K = K; p.ldc = ldc; p.epi = TC_EPI_F32; p.diag_n = n;
+  p.staged = (((uintptr_t)C & 15) == 0 && ldc % 4 == 0) ? 1 : 0;
+  return bn == 256 ? launch_tc<256, false>(ma, mw, p, n_sms, stream) : launch_tc<128, false>(ma, mw, p, n_sms, stream);
 }
 
 extern "C" int ie_gemm_tcgen05(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc,

@@ -160,21 +160,36 @@ moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int n_experts, int til
     if (e >= 0 && e < n_experts) atomicAdd(&count[e], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int pos = 0, nt = 0;
-    for (int e = 0; e < n_experts; ++e) {
-      offset[e] = pos;
-      for (int r = 0; r < count[e] && nt < max_tiles; r += tile_rows, ++nt) {
-        tiles[4 * nt] = e;
-        tiles[4 * nt + 1] = pos + r;
-        tiles[4 * nt + 2] = min(tile_rows, count[e] - r);
-        tiles[4 * nt + 3] = 0;
+  // a lane an expert: where its pairs and its tiles start is a sum over the experts before (one thread that walked all experts
+  // and wrote every tile was most of the kernel's time)
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int pos0 = 0, nt0 = 0;
+    for (int e0 = 0; e0 < n_experts; e0 += 32) {
+      const int e = e0 + lane;
+      const int n = e < n_experts ? count[e] : 0, nt = (n + tile_rows - 1) / tile_rows;
+      int pos = n, at = nt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, pos, o), b = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) {
+          pos += a;
+          at += b;
+        }
       }
-      pos += count[e];
+      const int all_pos = __shfl_sync(0xffffffffu, pos, 31), all_nt = __shfl_sync(0xffffffffu, at, 31);
+      pos += pos0 - n;
+      at += nt0 - nt;
+      if (e < n_experts) offset[e] = pos;
+      for (int i = 0; i < nt && at + i < max_tiles; ++i)
+        reinterpret_cast<int4*>(tiles)[at + i] = make_int4(e, pos + i * tile_rows, min(tile_rows, n - i * tile_rows), 0);
+      pos0 += all_pos;
+      nt0 += all_nt;
     }
-    const int n_tiles = nt;
-    for (; nt < max_tiles; ++nt) tiles[4 * nt] = tiles[4 * nt + 1] = tiles[4 * nt + 2] = tiles[4 * nt + 3] = 0;
-    tiles[3] = n_tiles;
+    nt0 = min(nt0, max_tiles);
+    for (int i = nt0 + lane; i < max_tiles; i += 32) reinterpret_cast<int4*>(tiles)[i] = make_int4(0, 0, 0, 0);
+    __syncwarp();
+    if (lane == 0) tiles[3] = nt0;
   }
   __syncthreads();
   for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
@@ -194,15 +209,15 @@ extern "C" int ie_moe_sort(const int* ids, int n_pairs, int n_experts, int tile_
 // ------------------------------------------------------------------ rows in sorted order
 // out[pos] = x[sorted[pos] / top] in 16-byte pieces: what the grouped product on tcgen05 reads, whose rows must lie in a row
 __global__ void moe_gather_kernel(const bf16* __restrict__ x, int x_stride, bf16* __restrict__ out, const int* __restrict__ sorted,
-                                  int top, int pieces, size_t total) {
+                                  int top, int pieces, int n_pairs) {
   pdl_trigger();
   pdl_wait();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const size_t pos = i / pieces;
-  const int c = (int)(i - pos * pieces) * 8;
-  *reinterpret_cast<uint4*>(out + pos * pieces * 8 + c) =
-      *reinterpret_cast<const uint4*>(x + (size_t)(sorted[pos] / top) * x_stride + c);
+  // a row of threads a pair
+  const int pos = blockIdx.x * blockDim.y + threadIdx.y;
+  if (pos >= n_pairs) return;
+  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(sorted[pos] / top) * x_stride);
+  uint4* dst = reinterpret_cast<uint4*>(out) + (size_t)pos * pieces;
+  for (int c = threadIdx.x; c < pieces; c += blockDim.x) dst[c] = src[c];
 }
 
 extern "C" int ie_moe_gather(const void* x, int x_stride, void* out, const int* sorted, int top, int n_pairs, int d,
@@ -210,9 +225,8 @@ extern "C" int ie_moe_gather(const void* x, int x_stride, void* out, const int* 
   if (n_pairs <= 0) return IE_OK;
   if (top <= 0 || d <= 0 || d % 8 || x_stride % 8) return IE_BAD_SIZE;
   if (((uintptr_t)x | (uintptr_t)out) & 15) return IE_BAD_ALIGN;
-  const size_t total = (size_t)n_pairs * (d / 8);
-  return launch_k(moe_gather_kernel, (unsigned)((total + 255) / 256), 256, 0, stream, (const bf16*)x, x_stride, (bf16*)out, sorted,
-                  top, d / 8, total);
+  return launch_k(moe_gather_kernel, (unsigned)((n_pairs + 3) / 4), dim3(64, 4), 0, stream, (const bf16*)x, x_stride, (bf16*)out, sorted,
+                  top, d / 8, n_pairs);
 }
 
 // ------------------------------------------------------------------ grouped product

@@ -51,9 +51,146 @@ __global__ void outnorm_accumulate_kernel(float* __restrict__ residual, const TY
   }
 }
 
+// Rows on 16 bytes, up to 8,192 wide: a thread keeps 8 columns at a time in registers, all loads 16 bytes a lane and in flight together
+// (element by element a row is three trips to memory, one after the other: 2,048 rows of 2,048 took 20 us, ONV_MEASURED here).
+// COMBINE: the row is not there yet; it is the weighted sum of a mixture's chosen experts plus the shared expert's,
+// sum over r of weights[t, r] * y[t * top + r] (r upward) + gate[t] * shared[t], which then never goes to memory.
+__device__ __forceinline__ void on_load8(const float* p, float (&v)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void on_load8(const bf16* p, float (&v)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __bfloat1622float2(h[e]);
+    v[2 * e] = f.x;
+    v[2 * e + 1] = f.y;
+  }
+}
+__device__ __forceinline__ void on_store8(float* p, const float (&v)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void on_store8(bf16* p, const float (&v)[8]) {
+  uint4 raw;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+  *reinterpret_cast<uint4*>(p) = raw;
+}
+constexpr int ON_THREADS = 256;
+struct OnCombine {
+  const float* weights;     // [n, top]
+  const float* gate;        // [n] or null
+  int top;
+};
+
+template <typename TY, typename TS, typename TW, typename TA, int PIECES, bool COMBINE>
+__global__ void __launch_bounds__(ON_THREADS) outnorm_rows_kernel(float* __restrict__ residual, const TY* __restrict__ y, int y_stride,
+                                                                  OnCombine mix, const TS* __restrict__ shared_out, int shared_stride,
+                                                                  const TW* __restrict__ gain, TA* __restrict__ next_in, int d, float eps) {
+  __shared__ float red[33];
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x;
+  float v[PIECES][8], ss = 0.f;
+#pragma unroll
+  for (int q = 0; q < PIECES; ++q) {
+    const int i = (q * ON_THREADS + threadIdx.x) * 8;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[q][e] = 0.f;
+    if (i < d) {
+      if (COMBINE) {
+        const float* w = mix.weights + (size_t)row * mix.top;
+        for (int r = 0; r < mix.top; ++r) {
+          float t[8];
+          on_load8(y + ((size_t)row * mix.top + r) * d + i, t);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[q][e] = fmaf(w[r], t[e], v[q][e]);
+        }
+        if (shared_out != nullptr) {
+          const float g = mix.gate != nullptr ? mix.gate[row] : 0.f;
+          float t[8];
+          on_load8(shared_out + (size_t)row * shared_stride + i, t);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[q][e] = fmaf(g, t[e], v[q][e]);
+        }
+      } else {
+        on_load8(y + (size_t)row * y_stride + i, v[q]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss = fmaf(v[q][e], v[q][e], ss);
+  }
+  const float rms = sqrtf(block_sum(ss, red) / (float)d + eps);
+#pragma unroll
+  for (int q = 0; q < PIECES; ++q) {
+    const int i = (q * ON_THREADS + threadIdx.x) * 8;
+    if (i < d) {
+      float x[8], g[8];
+      on_load8(residual + (size_t)row * d + i, x);
+      on_load8(gain + i, g);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] += (v[q][e] / rms) * g[e];
+      on_store8(residual + (size_t)row * d + i, x);
+      if (next_in != nullptr) on_store8(next_in + (size_t)row * d + i, x);
+    }
+  }
+}
+
+template <typename TY, typename TS, typename TW, bool COMBINE>
+static int launch_outnorm_rows(float* residual, const void* y, int y_stride, OnCombine mix, const void* shared_out, int shared_stride,
+                               const void* gain, void* next_in, int next_dtype, int n_rows, int d, float eps, cudaStream_t stream) {
+  const int pieces = (d / 8 + ON_THREADS - 1) / ON_THREADS;
+#define ONR(TA, P)                                                                                                          \
+  return launch_k(outnorm_rows_kernel<TY, TS, TW, TA, P, COMBINE>, n_rows, ON_THREADS, 0, stream, residual, (const TY*)y, y_stride, \
+                  mix, (const TS*)shared_out, shared_stride, (const TW*)gain, (TA*)next_in, d, eps)
+  if (next_in == nullptr || next_dtype == IE_BF16) {
+    if (pieces <= 1) ONR(bf16, 1);
+    if (pieces == 2) ONR(bf16, 2);
+    ONR(bf16, 4);
+  }
+  if (next_dtype != IE_F32) return IE_BAD_DTYPE;
+  if (pieces <= 1) ONR(float, 1);
+  if (pieces == 2) ONR(float, 2);
+  ONR(float, 4);
+#undef ONR
+}
+
+static bool outnorm_rows_fit(const void* residual, const void* y, int y_stride, const void* gain, const void* next_in, int d) {
+  return d % 8 == 0 && d <= 8 * ON_THREADS * 4 && y_stride % 8 == 0 &&
+         (((uintptr_t)residual | (uintptr_t)y | (uintptr_t)gain | (uintptr_t)next_in) & 15) == 0;
+}
+
+// residual += norm(sum_r weights[t, r] y[t top + r] + gate[t] shared[t]); rows on 16 bytes, d a multiple of 8 and
+// at most 8,192
+extern "C" int ie_moe_combine_outnorm(float* residual, const float* y, const float* weights, const float* gate, const void* shared_out,
+                                      int shared_dtype, int shared_stride, const void* gain, int gain_dtype, void* next_in,
+                                      int next_dtype, int n_rows, int d, int top, float eps, cudaStream_t stream) {
+  if (n_rows <= 0) return IE_OK;
+  if (top <= 0 || !outnorm_rows_fit(residual, y, d, gain, next_in, d)) return IE_BAD_SIZE;
+  if (shared_out != nullptr && (shared_stride % 8 || ((uintptr_t)shared_out & 15))) return IE_BAD_ALIGN;
+  const OnCombine mix = {weights, gate, top};
+#define ONC(TS, TW)                                                                                                          \
+  return launch_outnorm_rows<float, TS, TW, true>(residual, y, d, mix, shared_out, shared_stride, gain, next_in, next_dtype, \
+                                                  n_rows, d, eps, stream)
+  const bool shared_f32 = shared_out == nullptr || shared_dtype == IE_F32;
+  if (shared_f32 && gain_dtype == IE_F32) ONC(float, float);
+  if (shared_f32 && gain_dtype == IE_BF16) ONC(float, bf16);
+  if (shared_dtype == IE_BF16 && gain_dtype == IE_F32) ONC(bf16, float);
+  if (shared_dtype == IE_BF16 && gain_dtype == IE_BF16) ONC(bf16, bf16);
+#undef ONC
+  return IE_BAD_DTYPE;
+}
+
 template <typename TY, typename TW>
 static int launch_outnorm(float* residual, const void* y, int y_stride, const void* gain, void* next_in, int next_dtype,
                           int n_rows, int d, float eps, cudaStream_t stream) {
+  if (outnorm_rows_fit(residual, y, y_stride, gain, next_in, d))
+    return launch_outnorm_rows<TY, TY, TW, false>(residual, y, y_stride, OnCombine{nullptr, nullptr, 0}, nullptr, 0, gain, next_in,
+                                                  next_dtype, n_rows, d, eps, stream);
   const size_t smem = (size_t)d * sizeof(float);
   if (smem > 200 * 1024) return IE_BAD_SIZE;
   const int threads = d >= 2048 ? 512 : (d >= 512 ? 256 : 128);
@@ -225,6 +362,89 @@ causal_conv_kernel(const TA* __restrict__ x, int x_stride, const TW* __restrict_
   }
 }
 
+// bfloat16 rows on 16 bytes, filters of up to four taps: a thread takes 8 channels and 8 tokens in a row and keeps the inputs of the
+// filter's length in registers, so a row is read once, 16 bytes a lane (the kernel above reads two bytes a lane and every row
+// `taps` times).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 70 us, CV_MEASURED.
+#define CV_CH 8
+#define CV_RUN 8
+template <typename TW, int TAPS>
+__global__ void __launch_bounds__(256)
+causal_conv_vec_kernel(const bf16* __restrict__ x, int x_stride, const TW* __restrict__ w, const TW* __restrict__ bias, bf16* __restrict__ state,
+                       long long state_slot_stride, bf16* __restrict__ out, int out_stride, const int* __restrict__ q_start,
+                       const int* __restrict__ slots, int channels, int activation, int write_state) {
+  pdl_trigger();
+  pdl_wait();
+  const int c = (blockIdx.x * 32 + threadIdx.x) * CV_CH;
+  const int req = blockIdx.y;
+  const int q0 = q_start[req], q1 = q_start[req + 1];
+  const int t_lo = q0 + blockIdx.z * CONV_CHUNK + threadIdx.y * CV_RUN, t_hi = min(q1, t_lo + CV_RUN);
+  if (q0 + (int)blockIdx.z * CONV_CHUNK >= q1 && blockIdx.z > 0) return;     // a shorter request than the step's longest
+  const int slot = IE_SLOT(slots[req]);
+  const bool live = c < channels;
+  bf16* st = (slot >= 0 && live) ? state + (size_t)slot * state_slot_stride + c : nullptr;   // element i at st[i * channels]
+  constexpr int KEEP = TAPS - 1;
+  // the input of token `src` (from the state where the step does not hold it; zeros without a state)
+  auto row = [&](int src) -> uint4 {
+    if (src >= q0) return *reinterpret_cast<const uint4*>(x + (size_t)src * x_stride + c);
+    if (st != nullptr) return *reinterpret_cast<const uint4*>(st + (size_t)(KEEP - (q0 - src)) * channels);
+    return make_uint4(0u, 0u, 0u, 0u);
+  };
+  auto widen = [](const uint4& raw, float (&v)[CV_CH]) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __bfloat1622float2(h[e]);
+      v[2 * e] = f.x;
+      v[2 * e + 1] = f.y;
+    }
+  };
+  if (live && t_lo < t_hi) {
+    float wv[TAPS][CV_CH], b[CV_CH], in[TAPS][CV_CH];
+#pragma unroll
+    for (int e = 0; e < CV_CH; ++e) {
+      b[e] = bias != nullptr ? to_f32(bias[c + e]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) wv[j][e] = to_f32(w[(size_t)(c + e) * TAPS + j]);
+    }
+    uint4 raw[KEEP + CV_RUN];
+#pragma unroll
+    for (int i = 0; i < KEEP + CV_RUN; ++i) {
+      const int src = t_lo - KEEP + i;
+      raw[i] = src < t_hi ? row(src) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) widen(raw[j], in[j]);
+#pragma unroll
+    for (int i = 0; i < CV_RUN; ++i) {
+      widen(raw[KEEP + i], in[(KEEP + i) % TAPS]);
+      uint4 o;
+      __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+      for (int e = 0; e < CV_CH; e += 2) {
+        float acc[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          acc[q] = b[e + q];
+#pragma unroll
+          for (int j = 0; j < TAPS; ++j) acc[q] = fmaf(wv[j][e + q], in[(i + j) % TAPS][e + q], acc[q]);
+          if (activation == 1) acc[q] = acc[q] / (1.f + expf(-acc[q]));
+        }
+        op[e / 2] = __floats2bfloat162_rn(acc[0], acc[1]);
+      }
+      if (t_lo + i < t_hi) *reinterpret_cast<uint4*>(out + (size_t)(t_lo + i) * out_stride + c) = o;
+    }
+  }
+  if (blockIdx.z > 0) return;
+  __syncthreads();                          // the state has been read: only a request's first chunk looks at it
+  if (write_state && st != nullptr && threadIdx.y == 0) {
+    uint4 nv[KEEP > 0 ? KEEP : 1];
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) nv[i] = row(q1 - KEEP + i);
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) *reinterpret_cast<uint4*>(st + (size_t)i * channels) = nv[i];
+  }
+}
+
 extern "C" int ie_causal_conv(const void* x, int x_stride, const void* w, const void* bias, int w_dtype, void* state,
                               long long state_slot_stride, void* out, int out_stride, const int* q_start,
                               const int* slots, int n_requests, int channels, int taps, int activation,
@@ -234,6 +454,23 @@ extern "C" int ie_causal_conv(const void* x, int x_stride, const void* w, const 
   const int chunks = (max_q_len + CONV_CHUNK - 1) / CONV_CHUNK;       // of the step's longest request
   if (chunks > 65535) return IE_BAD_SIZE;
   dim3 grid((channels + CONV_CH - 1) / CONV_CH, n_requests, chunks), block(CONV_CH, CONV_TL);
+  const bool vec = act_dtype == IE_BF16 && taps >= 2 && taps <= 4 && channels % CV_CH == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 &&
+                   state_slot_stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)state) & 15) == 0;
+#define CV_GO(TW, TAPS)                                                                                            \
+  return launch_k(causal_conv_vec_kernel<TW, TAPS>, dim3((channels + 32 * CV_CH - 1) / (32 * CV_CH), n_requests, chunks),   \
+                  dim3(32, CONV_CHUNK / CV_RUN), 0, stream, (const bf16*)x, x_stride, (const TW*)w, (const TW*)bias, \
+                  (bf16*)state, state_slot_stride, (bf16*)out, out_stride, q_start, slots, channels, activation, write_state)
+  if (vec && w_dtype == IE_BF16) {
+    if (taps == 4) CV_GO(bf16, 4);
+    if (taps == 3) CV_GO(bf16, 3);
+    CV_GO(bf16, 2);
+  }
+  if (vec && w_dtype == IE_F32) {
+    if (taps == 4) CV_GO(float, 4);
+    if (taps == 3) CV_GO(float, 3);
+    CV_GO(float, 2);
+  }
+#undef CV_GO
 #define CONV_GO(TA, TW)                                                                                          \
   return launch_k(causal_conv_kernel<TA, TW>, grid, block, 0, stream, (const TA*)x, x_stride, (const TW*)w,      \
                   (const TW*)bias, (TA*)state, state_slot_stride, (TA*)out, out_stride, q_start, slots, channels, \
@@ -320,22 +557,120 @@ linear_recurrence_kernel(const TA* __restrict__ u, int u_stride, const TA* __res
   if (write_state) state[(size_t)slot * width + c] = S;
 }
 
+// Many tokens: the chain above walks a request's tokens in one thread a channel (2,048 tokens of 2,048 channels: 1,042 us, 16
+// blocks, each token's exponentials in the chain).  Here a block takes 16 channels and LS_SLICES runs of LS_TOK tokens; a
+// thread forms the decays and inputs of its run, runs it from a state of zero, and the runs' (sum of log a, end state)
+// pairs are put together by a scan in shared memory; then the run goes again from the state it really starts with.
+// 2,048 tokens of 2,048 channels: LS_MEASURED.
+#define LS_CH 16
+#define LS_SLICES 64
+#define LS_TOK 8
+#define LS_MIN_TOKENS 64      // of the longest request of a step (64 tokens of one request: LS_AT_64)
+template <typename TA, typename TW>
+__global__ void __launch_bounds__(LS_CH * LS_SLICES)
+linear_recurrence_runs_kernel(const TA* __restrict__ u, int u_stride, const TA* __restrict__ y_pre, int y_stride,
+                              const float* __restrict__ r_pre, const float* __restrict__ i_pre, int g_stride,
+                              const TW* __restrict__ r_bias, const TW* __restrict__ i_bias, const TW* __restrict__ lam,
+                              float* __restrict__ state, TA* __restrict__ out, int out_stride,
+                              const int* __restrict__ q_start, const int* __restrict__ slots, int width,
+                              float decay_scale, float out_scale, int write_state) {
+  __shared__ float s_end[LS_SLICES][LS_CH], s_log[LS_SLICES][LS_CH];
+  pdl_trigger();
+  pdl_wait();
+  const int ch = threadIdx.x % LS_CH, run = threadIdx.x / LS_CH;
+  const int c = blockIdx.x * LS_CH + ch, req = blockIdx.y;
+  const bool live = c < width;
+  const int q0 = q_start[req], q1 = q_start[req + 1];
+  const int slot = IE_SLOT(slots[req]);
+  if (slot < 0) {
+    for (int t = q0 + run; t < q1 && live; t += LS_SLICES) out[(size_t)t * out_stride + c] = from_f32<TA>(0.f);
+    return;
+  }
+  const float rb = live ? to_f32(r_bias[c]) : 0.f, ib = live ? to_f32(i_bias[c]) : 0.f;
+  const float rate = live ? -decay_scale * softplus_f(to_f32(lam[c])) : 0.f;
+  float carry = live ? state[(size_t)slot * width + c] : 0.f;
+  for (int base = q0; base < q1; base += LS_SLICES * LS_TOK) {
+    const int t0 = base + run * LS_TOK;
+    const int nt = live ? max(0, min(LS_TOK, q1 - t0)) : 0;
+    // a token's step is S + (m S + in) while its bit in `near` is set (a above one half, m = a - 1), else a S + in with m = a;
+    // a token that is not there leaves S as it is
+    float m[LS_TOK], in[LS_TOK], L = 0.f, E = 0.f;
+    unsigned near = 0;
+#pragma unroll
+    for (int k = 0; k < LS_TOK; ++k) {
+      const size_t t = (size_t)(k < nt ? t0 + k : q0);
+      m[k] = live ? r_pre[t * g_stride + c] : 0.f;
+      in[k] = live ? i_pre[t * g_stride + c] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < LS_TOK; ++k) {
+      if (k < nt) {
+        const float log_a = rate * sigmoid_f(m[k] + rb);
+        in[k] = sqrtf(-expm1f(2.f * log_a)) * (sigmoid_f(in[k] + ib) * to_f32(u[(size_t)(t0 + k) * u_stride + c]));
+        const bool close = log_a > -0.6931472f;
+        m[k] = close ? expm1f(log_a) : expf(log_a);
+        near |= (close ? 1u : 0u) << k;
+        L += log_a;
+      } else {
+        m[k] = in[k] = 0.f;
+        near |= 1u << k;
+      }
+      const float x = fmaf(m[k], E, in[k]);
+      E = ((near >> k) & 1u) ? E + x : x;
+    }
+    s_end[run][ch] = E;
+    s_log[run][ch] = L;
+    __syncthreads();
+#pragma unroll
+    for (int o = 1; o < LS_SLICES; o <<= 1) {
+      float pe = 0.f, pl = 0.f;
+      if (run >= o) {
+        pe = s_end[run - o][ch];
+        pl = s_log[run - o][ch];
+      }
+      __syncthreads();
+      if (run >= o) {
+        s_end[run][ch] = E = lru_step(pe, L, E);
+        s_log[run][ch] = L = L + pl;
+      }
+      __syncthreads();
+    }
+    float S = run == 0 ? carry : lru_step(carry, s_log[run - 1][ch], s_end[run - 1][ch]);
+    carry = lru_step(carry, s_log[LS_SLICES - 1][ch], s_end[LS_SLICES - 1][ch]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < LS_TOK; ++k) {
+      const float x = fmaf(m[k], S, in[k]);
+      S = ((near >> k) & 1u) ? S + x : x;
+      if (k < nt)
+        out[(size_t)(t0 + k) * out_stride + c] =
+            from_f32<TA>(out_scale * S * gelu_tanh_f(to_f32(y_pre[(size_t)(t0 + k) * y_stride + c])));
+    }
+  }
+  if (write_state && live && run == 0) state[(size_t)slot * width + c] = carry;
+}
+
+// max_q_len: tokens of the step's longest request (0: not known, token after token)
 extern "C" int ie_linear_recurrence(const void* u, int u_stride, const void* y_pre, int y_stride, const float* r_pre,
                                     const float* i_pre, int g_stride, const void* r_bias, const void* i_bias,
                                     const void* lam, int w_dtype, float* state, void* out, int out_stride,
                                     const int* q_start, const int* slots, int n_requests, int width,
-                                    float decay_scale, float out_scale, int write_state, int act_dtype,
+                                    float decay_scale, float out_scale, int write_state, int act_dtype, int max_q_len,
                                     cudaStream_t stream) {
   if (n_requests <= 0 || width <= 0) return IE_OK;
-  dim3 grid((width + 127) / 128, n_requests);
+  dim3 grid((width + 127) / 128, n_requests), run_grid((width + LS_CH - 1) / LS_CH, n_requests);
 #define LRU_GO(TA, TW)                                                                                             \
+  if (max_q_len >= LS_MIN_TOKENS)                                                                                  \
+    return launch_k(linear_recurrence_runs_kernel<TA, TW>, run_grid, LS_CH * LS_SLICES, 0, stream, (const TA*)u, u_stride, \
+                    (const TA*)y_pre, y_stride, r_pre, i_pre, g_stride, (const TW*)r_bias, (const TW*)i_bias,       \
+                    (const TW*)lam, state, (TA*)out, out_stride, q_start, slots, width, decay_scale, out_scale, write_state); \
   return launch_k(linear_recurrence_kernel<TA, TW>, grid, 128, 0, stream, (const TA*)u, u_stride, (const TA*)y_pre, \
                   y_stride, r_pre, i_pre, g_stride, (const TW*)r_bias, (const TW*)i_bias, (const TW*)lam, state,    \
                   (TA*)out, out_stride, q_start, slots, width, decay_scale, out_scale, write_state)
-  if (act_dtype == IE_F32 && w_dtype == IE_F32) LRU_GO(float, float);
-  if (act_dtype == IE_F32 && w_dtype == IE_BF16) LRU_GO(float, bf16);
-  if (act_dtype == IE_BF16 && w_dtype == IE_F32) LRU_GO(bf16, float);
-  if (act_dtype == IE_BF16 && w_dtype == IE_BF16) LRU_GO(bf16, bf16);
+  if (act_dtype == IE_F32 && w_dtype == IE_F32) { LRU_GO(float, float); }
+  if (act_dtype == IE_F32 && w_dtype == IE_BF16) { LRU_GO(float, bf16); }
+  if (act_dtype == IE_BF16 && w_dtype == IE_F32) { LRU_GO(bf16, float); }
+  if (act_dtype == IE_BF16 && w_dtype == IE_BF16) { LRU_GO(bf16, bf16); }
 #undef LRU_GO
   return IE_BAD_DTYPE;
 }

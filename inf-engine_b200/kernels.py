@@ -91,14 +91,18 @@ def core():
         lib.ie_headnorm_kv_write.argtypes = [P, P, P, I, I, I, P, P, I, F, P, P, P, I, I, I, I, I, I, I, I, P]
         lib.ie_gemm_simt.argtypes = [P, I, P, I, P, I, I, I, I, I, I, I, P]
         lib.ie_gemm_simt_batched.argtypes = [P, I, P, I, P, I, I, I, I, I, I, I, I, L, L, L, P]
+        lib.ie_gemm_diag_rows.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P]
+        lib.ie_gemm_diag_rows.restype = c_int
         lib.ie_gemm_rowdot.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P]
         lib.ie_cast_rows.argtypes = [P, P, I, I, I, P]
         lib.ie_outnorm_accumulate.argtypes = [P, P, I, I, P, I, P, I, I, I, F, P]
+        lib.ie_moe_combine_outnorm.argtypes = [P, P, P, P, P, I, I, P, I, P, I, I, I, I, F, P]
+        lib.ie_moe_combine_outnorm.restype = c_int
         lib.ie_outnorm_accumulate_norm.argtypes = [P, P, I, I, P, I, F, P, I, F, P, I, I, I, P]
         lib.ie_outnorm_accumulate_norm.restype = c_int
         lib.ie_causal_conv.argtypes = [P, I, P, P, I, P, L, P, I, P, P, I, I, I, I, I, I, I, P]
         lib.ie_attention_rows.argtypes = [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, I, P, I, P, I, I, F, I, I, I, P, F, P, I, P]
-        lib.ie_linear_recurrence.argtypes = [P, I, P, I, P, P, I, P, P, P, I, P, P, I, P, P, I, I, F, F, I, I, P]
+        lib.ie_linear_recurrence.argtypes = [P, I, P, I, P, P, I, P, P, P, I, P, P, I, P, P, I, I, F, F, I, I, I, P]
         lib.ie_rownorm_rotate_write.argtypes = [P, P, P, I, I, I, P, P, P, P, P, I, F, P, I, P, P, P, P, I, I, I, I, I, I, I, P]
         lib.ie_moe_route.argtypes = [P, I, P, I, P, P, P, I, I, I, I, I, F, F, I, I, I, P]
         lib.ie_moe_gather.argtypes = [P, I, P, P, I, I, I, P]
@@ -413,6 +417,29 @@ def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
            f"gemm_simt_batched({a.dtype},{w.dtype}, blocks={blocks})")
 
 
+DIAG_FEW_ROWS = 16      # up to here a warp an output column beats tiles of 64 rows
+
+
+def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """``gemm_simt_batched`` by the kernel that suits the rows: a warp an output for a few, the tcgen05 tensor cores for
+    bfloat16 operands from a tile of 128 rows on (their products are exact in float32, the sums float32), tiles on CUDA
+    cores else."""
+    blocks, n, k = w.shape
+    m = a.shape[0]
+    assert a.shape[1] == blocks * k and out.shape == (m, blocks * n) and out.dtype is torch.float32
+    assert a.stride(1) == 1 and w.is_contiguous() and out.stride(1) == 1
+    aligned = a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+    if m <= DIAG_FEW_ROWS and k % 4 == 0 and a.stride(0) % 4 == 0 and aligned:
+        _check(core().ie_gemm_diag_rows(_ptr(a), dtype_code(a.dtype), _ptr(w), dtype_code(w.dtype), _ptr(out), m, blocks, n, k,
+                                        a.stride(0), out.stride(0), _stream()), f"gemm_diag_rows(blocks={blocks}, n={n}, k={k})")
+    elif (m >= 128 and a.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and n % 128 == 0 and aligned
+          and gemm_tcgen05_supports(m, n, k, a.stride(0), k)):
+        _check(tcgen05_library().ie_gemm_tcgen05_diag(_ptr(a), _ptr(w), _ptr(out), m, blocks, n, k, a.stride(0), out.stride(0),
+                                                      sm_count(), _stream()), f"gemm_tcgen05_diag(blocks={blocks}, n={n}, k={k})")
+    else:
+        gemm_simt_batched(a, w, out)
+
+
 # ------------------------------------------------------------- norm on a sublayer's output, state along a sequence
 def cast_rows(x: torch.Tensor, out: torch.Tensor) -> None:
     """out = x (float32 rows) in out's type."""
@@ -431,6 +458,28 @@ def outnorm_accumulate(residual: torch.Tensor, y: torch.Tensor, gain: torch.Tens
                                         dtype_code(gain.dtype), _ptr(next_in),
                                         dtype_code(next_in.dtype) if next_in is not None else IE_BF16, n, d, float(eps),
                                         _stream()), "outnorm_accumulate")
+
+
+def moe_combine_outnorm_supports(residual: torch.Tensor, shared_out: torch.Tensor | None) -> bool:
+    d = residual.shape[1]
+    return (d % 8 == 0 and d <= 8192 and residual.data_ptr() % 16 == 0
+            and (shared_out is None or (shared_out.stride(0) % 8 == 0 and shared_out.data_ptr() % 16 == 0)))
+
+
+def moe_combine_outnorm(residual: torch.Tensor, y: torch.Tensor, weights: torch.Tensor, gate: torch.Tensor | None,
+                        shared_out: torch.Tensor | None, gain: torch.Tensor, eps: float, next_in: torch.Tensor | None = None) -> None:
+    """``moe_combine`` and ``outnorm_accumulate`` of its rows in one kernel (where ``moe_combine_outnorm_supports``)."""
+    n, top = weights.shape
+    d = residual.shape[1]
+    assert residual.dtype is torch.float32 and residual.is_contiguous() and residual.shape[0] == n
+    assert y.dtype is torch.float32 and y.is_contiguous() and y.shape == (n * top, d) and weights.is_contiguous()
+    assert shared_out is None or shared_out.stride(1) == 1
+    assert gain.shape == (d,) and (next_in is None or (next_in.is_contiguous() and next_in.shape == (n, d)))
+    _check(core().ie_moe_combine_outnorm(_ptr(residual), _ptr(y), _ptr(weights), _ptr(gate), _ptr(shared_out),
+                                         dtype_code(shared_out.dtype) if shared_out is not None else IE_F32,
+                                         shared_out.stride(0) if shared_out is not None else 0, _ptr(gain), dtype_code(gain.dtype),
+                                         _ptr(next_in), dtype_code(next_in.dtype) if next_in is not None else IE_BF16, n, d, top,
+                                         float(eps), _stream()), "moe_combine_outnorm")
 
 
 def outnorm_accumulate_norm(residual: torch.Tensor, y: torch.Tensor, gain: torch.Tensor, eps: float,
@@ -474,11 +523,12 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
 def linear_recurrence(u: torch.Tensor, y_pre: torch.Tensor, r_pre: torch.Tensor, i_pre: torch.Tensor,
                       r_bias: torch.Tensor, i_bias: torch.Tensor, lam: torch.Tensor, state: torch.Tensor,
                       out: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, n_requests: int,
-                      decay_scale: float, out_scale: float = 1.0, write_state: bool = True) -> None:
+                      decay_scale: float, out_scale: float = 1.0, write_state: bool = True, max_q_len: int = 0) -> None:
     """The real-gated linear recurrent unit over each request's tokens of the step, per channel: r = sigmoid(r_pre +
     r_bias), i = sigmoid(i_pre + i_bias), a = exp(-decay_scale * r * softplus(lam)), S <- a S + sqrt(1 - a^2) i u,
     out = out_scale * S * gelu_tanh(y_pre).  ``r_pre``/``i_pre`` float32 (columns of one buffer), ``state`` float32
-    [slots, width]."""
+    [slots, width].  ``max_q_len``: tokens of the step's longest request; many are taken in runs side by side (0: one token
+    after another)."""
     n, width = u.shape
     assert u.stride(1) == 1 and y_pre.stride(1) == 1 and y_pre.dtype == u.dtype == out.dtype and out.stride(1) == 1
     assert r_pre.dtype is torch.float32 and i_pre.dtype is torch.float32 and r_pre.stride(0) == i_pre.stride(0)
@@ -489,7 +539,7 @@ def linear_recurrence(u: torch.Tensor, y_pre: torch.Tensor, r_pre: torch.Tensor,
                                        r_pre.stride(0), _ptr(r_bias), _ptr(i_bias), _ptr(lam), dtype_code(lam.dtype),
                                        _ptr(state), _ptr(out), out.stride(0), _ptr(q_start), _ptr(slots), n_requests,
                                        width, float(decay_scale), float(out_scale), 1 if write_state else 0,
-                                       dtype_code(u.dtype), _stream()), f"linear_recurrence(width={width})")
+                                       dtype_code(u.dtype), int(max_q_len), _stream()), f"linear_recurrence(width={width})")
 
 
 def rownorm_rotate_write(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_bias, k_bias, v_bias, q_gain, k_gain,
@@ -843,6 +893,29 @@ def moe_gemm(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, sorted_pairs: to
                               float(limit), float(up_offset), float(cubic),
                               1 if c.shape[0] <= MOE_FEW_TOKENS * top else 0, _stream()),
            f"moe_gemm(n={n}, k={k}, {epi})")
+
+
+def moe_ring_supports(x: torch.Tensor, hidden: int, intermediate: int) -> bool:
+    """Whether ``moe_gemm_ring`` takes both products of experts of these sizes for the tokens ``x``."""
+    return (0 < x.shape[0] <= MOE_FEW_TOKENS and x.dtype is torch.bfloat16 and hidden % 256 == 0 and intermediate % 256 == 0
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+
+
+MOE_RING_ROWS = 16        # most rows of a tile of ``moe_gemm_ring``
+
+
+def moe_gemm_ring(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, sorted_pairs: torch.Tensor, tiles: torch.Tensor,
+                  top: int, gather: bool, scatter: bool, epi: str = "f32", act: tuple | None = None) -> None:
+    """``moe_gemm`` for at most 16 tokens in bfloat16: the chosen experts' weights through a ring of bulk copies, tiles of at
+    most ``MOE_RING_ROWS`` rows.  ``epi``: "f32" store, "silu_mul" with the activation ``act``, or "relu2"."""
+    _, n, k = w.shape
+    assert a.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and w.is_contiguous() and a.stride(1) == 1 and c.stride(1) == 1
+    assert a.shape[1] == k and c.shape[1] == (n // 2 if epi == "silu_mul" else n)
+    assert c.dtype is (torch.float32 if epi == "f32" else torch.bfloat16)
+    _check(stream_library().ie_moe_ring(_ptr(a), _ptr(w), _ptr(c), _ptr(sorted_pairs), _ptr(tiles), tiles.shape[0], n, k,
+                                        a.stride(0), c.stride(0), top, 1 if gather else 0, 1 if scatter else 0,
+                                        _EPI["glu" if epi == "silu_mul" else epi], sm_count(), *_act4(act), _stream()),
+           f"moe_gemm_ring(n={n}, k={k}, {epi})")
 
 
 def moe_gather(x: torch.Tensor, out: torch.Tensor, sorted_pairs: torch.Tensor, top: int) -> None:
@@ -1344,6 +1417,8 @@ def _bind_stream(lib):
     lib.ie_gemm_stream_tma_supports.argtypes = [I, I, I, I]
     lib.ie_gemm_stream_tma_supports.restype = c_int
     lib.ie_gemm_stream_tma_error.restype = c_int
+    lib.ie_moe_ring.argtypes = [P] * 5 + [I] * 10 + [F] * 4 + [P]
+    lib.ie_moe_ring.restype = c_int
     return lib
 
 
@@ -1454,6 +1529,8 @@ def tcgen05_library():
         lib.ie_gemm_tcgen05.restype = c_int
         lib.ie_gemm_tcgen05_act.argtypes = [c_void_p] * 3 + [c_int] * 10 + [c_float] * 4 + [c_void_p]
         lib.ie_gemm_tcgen05_act.restype = c_int
+        lib.ie_gemm_tcgen05_diag.argtypes = [P, P, P] + [I] * 7 + [P]
+        lib.ie_gemm_tcgen05_diag.restype = c_int
         lib.ie_gemm_tcgen05_grouped.argtypes = [c_void_p] * 5 + [c_int] * 10 + [c_float] * 4 + [c_void_p]
         lib.ie_gemm_tcgen05_grouped.restype = c_int
         lib.ie_gemm_tcgen05_tile_rows.restype = c_int

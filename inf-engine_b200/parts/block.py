@@ -141,9 +141,12 @@ class OutputNormBlock:
         self.mixer_norm.accumulate(residual, a, nxt)
         ctx.residual_cast = nxt
         if self.feedforward is not None:
-            m = self.feedforward.forward(self._input(residual, ctx), ctx)
+            # a mixture's weighted sum, the norm of it and the sum into the residual are one kernel
+            mixture = hasattr(self.feedforward, "forward_parts") and hasattr(self.ff_norm, "accumulate_mixture")
+            run = self.feedforward.forward_parts if mixture else self.feedforward.forward
+            m = run(self._input(residual, ctx), ctx)
             nxt = self._next_input(residual, not last)
-            self.ff_norm.accumulate(residual, m, nxt)
+            (self.ff_norm.accumulate_mixture if mixture else self.ff_norm.accumulate)(residual, m, nxt)
             ctx.residual_cast = nxt
         return residual, None
 

@@ -73,6 +73,16 @@ class RMSNorm:
         """residual += norm(y); ``next_in`` (activation type, optional) takes the new residual rows."""
         kernels.outnorm_accumulate(residual, y, self.gain, self.eps, next_in)
 
+    def accumulate_mixture(self, residual: torch.Tensor, parts, next_in: torch.Tensor | None = None) -> None:
+        """``accumulate`` of a mixture of experts that is not summed up yet (``RoutedExperts.forward_parts``)."""
+        y, weights, gate, shared = parts
+        if kernels.moe_combine_outnorm_supports(residual, shared):
+            kernels.moe_combine_outnorm(residual, y, weights, gate, shared, self.gain, self.eps, next_in)
+            return
+        out = self.rt.ws.take("moe_out", tuple(residual.shape), torch.float32)
+        kernels.moe_combine(y, weights, gate, shared, out)
+        self.accumulate(residual, out, next_in)
+
     def accumulate_then_norm(self, residual: torch.Tensor, y: torch.Tensor, next_norm, out_name: str = "normed"):
         """residual += norm(y), and in the same kernel the rows that ``next_norm`` (an RMS norm of this size) makes of
         the new residual; None when the two do not go together (the caller then runs them one after the other)."""

@@ -88,11 +88,11 @@ class GatedLinearRecurrence:
         kernels.causal_conv(proj[:, w:], self.conv_weight, self.conv_bias, conv_state.state, u, ctx.q_start, ctx.slots,
                             ctx.n_requests, activation=None, write_state=cache.write, max_q_len=ctx.max_q_len)
         gates = rt.ws.take("recurrence_gates", (n, 2 * w), torch.float32)
-        kernels.gemm_simt_batched(u, self.a_gate, gates[:, :w])
-        kernels.gemm_simt_batched(u, self.i_gate, gates[:, w:])
+        kernels.block_diagonal(u, self.a_gate, gates[:, :w])
+        kernels.block_diagonal(u, self.i_gate, gates[:, w:])
         kernels.linear_recurrence(u, proj[:, :w], gates[:, :w], gates[:, w:], self.a_bias, self.i_bias, self.lam,
                                   state.state, out, ctx.q_start, ctx.slots, ctx.n_requests, s.decay_scale, s.out_scale,
-                                  write_state=cache.write)
+                                  write_state=cache.write, max_q_len=ctx.max_q_len)
 
     def forward(self, x: torch.Tensor, ctx, cache) -> torch.Tensor:
         rt = self.rt

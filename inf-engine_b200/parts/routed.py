@@ -130,6 +130,15 @@ class RoutedExperts:
             kernels.gemm_tcgen05_grouped(xs, self.first, hidden, tiles, None, self.epi, act=self.act)
             kernels.gemm_tcgen05_grouped(hidden, self.down, y, tiles, sorted_pairs, "f32")
             return y, weights, gate
+        if (rt.act_dtype is torch.bfloat16 and self.first.dtype is torch.bfloat16 and self.down.dtype is torch.bfloat16
+                and kernels.moe_ring_supports(x, s.hidden, s.intermediate)):
+            rows = kernels.MOE_RING_ROWS
+            tiles = ws.take("moe_tiles", (kernels.moe_max_tiles(n_pairs, E, rows), 4), torch.int32)
+            kernels.moe_sort(ids, E, sorted_pairs, tiles, rows)
+            kernels.moe_gemm_ring(x, self.first, hidden, sorted_pairs, tiles, top, gather=True, scatter=False, epi=self.epi,
+                                  act=self.act)
+            kernels.moe_gemm_ring(hidden, self.down, y, sorted_pairs, tiles, top, gather=False, scatter=True)
+            return y, weights, gate
         tiles = ws.take("moe_tiles", (kernels.moe_max_tiles(n_pairs, E), 4), torch.int32)
         kernels.moe_sort(ids, E, sorted_pairs, tiles)
         kernels.moe_gemm(x, self.first, hidden, sorted_pairs, tiles, top, gather=True, scatter=False, epi=self.epi,
@@ -147,9 +156,14 @@ class RoutedExperts:
         y, weights, _ = self._run_experts(x)
         return y, weights, (self.shared.forward(x, ctx),) if self.shared is not None else ()
 
-    def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
+    def forward_parts(self, x: torch.Tensor, ctx):
+        """``(y, weights, gate, shared)`` for a caller that forms ``sum_r weights[n, r] * y[n * top + r] + gate[n] * shared[n]``
+        itself."""
         y, weights, gate = self._run_experts(x)
-        shared = self.shared.forward(x, ctx) if self.shared is not None else None
+        return y, weights, gate, self.shared.forward(x, ctx) if self.shared is not None else None
+
+    def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
+        y, weights, gate, shared = self.forward_parts(x, ctx)
         out = self.rt.ws.take("moe_out", (x.shape[0], self.spec.hidden), torch.float32)
         kernels.moe_combine(y, weights, gate, shared, out)
         return out

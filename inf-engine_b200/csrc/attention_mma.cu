@@ -67,7 +67,7 @@ struct MmaAttnParams {
   int q_stride, out_stride, table_stride;
   int n_heads, n_kv_heads, page_size, window;
   int page_shift;  // log2(page_size) when it is a power of two, else -1
-  int n_splits, split_keys;
+  int split_keys;  // decode: the split of the step's longest request
   float scale_log2;
   // decode with the position encoding and the cache write folded in (every request brings one token):
   // fuse bit 0: q arrives unrotated and is rotated as it is loaded; bit 1: the token's key and value arrive
@@ -580,7 +580,7 @@ __device__ __forceinline__ unsigned long long trace_now() {
 
 // -------------------------------------------------------------------- decode
 // A request brings at most 16 rows (q_len * group <= 16).  Block (x, kv head, request) has DC_WARPS warps,
-// each with one split of the keys: consecutive splits, so that a block covers DC_WARPS * split_keys keys.
+// each with one split of the request's keys: consecutive splits, so that a block covers DC_WARPS splits.
 // A warp keeps up to DC_STAGES key tiles in flight (a decode step is a matter of latency: few bytes per
 // warp, all of them wanted as early as possible).  The warps of a block add their partial results up
 // through shared memory, in ascending order of the splits.  A (request, kv head) that one block covers
@@ -666,13 +666,19 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   const int min_first = p.window > 0 ? max(0, ctx - p.window + 1) : 0;
   const int lo_all = (min_first / DC_KT) * DC_KT;
 
-  // splits that hold at least one key some row can see
-  const int s_first = lo_all / p.split_keys, s_last = max_lim / p.split_keys;
-  const int k_lo = max(split * p.split_keys, lo_all);
-  const int k_hi = min((split + 1) * p.split_keys, max_lim + 1);
-  const bool has_work = split >= s_first && split <= s_last && split < p.n_splits && n_pairs > 0;
-  // blocks that hold at least one such split
-  const int b_first = s_first / DC_WARPS, b_last = s_last / DC_WARPS;
+  // This request's own split: its visible keys over all the warps that the launch gives a (request, kv head), in whole tiles,
+  // at least 64 (or the launch's split, if that is shorter).  The launch is cut for the longest request of the step; with its
+  // split for all, a request of a quarter of those keys would leave three warps in four idle (64 requests of 250 to 1,750
+  // keys, heads of 64: 48.8 us a layer with one split for all, 44.0 with each its own).
+  const int span = max_lim + 1 - lo_all;
+  const int even = (span + (int)gridDim.x * DC_WARPS - 1) / ((int)gridDim.x * DC_WARPS);
+  const int split_keys = max(min(64, p.split_keys), (even + DC_KT - 1) / DC_KT * DC_KT);
+  const int s_last = (span - 1) / split_keys;
+  const int k_lo = lo_all + split * split_keys;
+  const int k_hi = min(k_lo + split_keys, max_lim + 1);
+  const bool has_work = split <= s_last && n_pairs > 0;
+  // blocks that hold at least one split
+  const int b_first = 0, b_last = s_last / DC_WARPS;
   const int n_active_blocks = b_last - b_first + 1;
   // A block without keys leaves at once and frees its slot.  It need not wait for the kernel ahead:
   // block 0 of every (request, kv head) always has keys and waits, so this kernel still ends after it.
@@ -932,7 +938,7 @@ static void fill(MmaAttnParams& p, const void* q, void* out, const void* kpool, 
   p.cluster_merge = 0;
   p.q_stride = q_stride; p.out_stride = out_stride; p.table_stride = table_stride;
   p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.page_size = page_size; p.window = window;
-  p.n_splits = 0; p.split_keys = 0; p.n_blocks = 0; p.scale_log2 = scale * LOG2E;
+  p.split_keys = 0; p.n_blocks = 0; p.scale_log2 = scale * LOG2E;
   p.fuse = 0; p.k_new = nullptr; p.v_new = nullptr; p.kv_stride = 0; p.cos_t = nullptr; p.sin_t = nullptr;
   p.positions = nullptr; p.slot_mapping = nullptr;
   p.score_bias = nullptr; p.bias_dists = 0; p.head_scale = nullptr;
@@ -1050,7 +1056,6 @@ static int decode_launch(MmaAttnParams& p, float* scratch, int n_requests, int n
                          int n_splits, int split_keys, cudaStream_t stream) {
   if (n_splits <= 0 || split_keys <= 0 || split_keys % DC_KT) return IE_BAD_SIZE;
   if ((uintptr_t)scratch & 15) return IE_BAD_ALIGN;
-  p.n_splits = n_splits;
   p.split_keys = split_keys;
   if ((long long)n_requests * n_kv_heads > IE_DECODE_TICKET_WORDS) return IE_BAD_SIZE;
   p.n_blocks = (n_splits + DC_WARPS - 1) / DC_WARPS;

@@ -122,16 +122,18 @@ extern "C" int ie_gemm_simt_batched(const void* A, int a_dtype, const void* W, i
   }
 }
 
-// The same for a few rows (decode tokens): a warp an output column, its lanes stride k four at a time with one sum per row, then a
-// tree over the lanes; the order is fixed by (n, k) alone.  The tile kernel gives 8 rows of 8 blocks of 256 x 256 to 32 thread
-// blocks that walk K alone, 16 stages of loads one after the other (28 us of a decode step; DR_MEASURED here).
-__device__ __forceinline__ float4 dr_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 dr_load4(const bf16* p) {
+// four neighbouring elements as float32
+__device__ __forceinline__ float4 rd_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 rd_load4(const bf16* p) {
   const uint2 raw = *reinterpret_cast<const uint2*>(p);
   const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
   const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
+
+// The same for a few rows (decode tokens): a warp an output column, its lanes stride k four at a time with one sum per row, then a
+// tree over the lanes; the order is fixed by (n, k) alone.  The tile kernel gives 8 rows of 8 blocks of 256 x 256 to 32 thread
+// blocks that walk K alone, 16 stages of loads one after the other (15.0 us; 4.9 here).
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(256) gemm_diag_rows_kernel(const TA* __restrict__ A, const TW* __restrict__ W, float* __restrict__ C,
                                                              int M, int cols, int n, int K, int lda, int ldc) {
@@ -145,10 +147,10 @@ __global__ void __launch_bounds__(256) gemm_diag_rows_kernel(const TA* __restric
   for (int m0 = 0; m0 < M; m0 += MR) {
     float acc[MR] = {};
     for (int k = lane * 4; k < K; k += 128) {
-      const float4 wv = dr_load4(w + k);
+      const float4 wv = rd_load4(w + k);
 #pragma unroll
       for (int r = 0; r < MR; ++r) {
-        const float4 x = dr_load4(a + (size_t)min(m0 + r, M - 1) * lda + k);
+        const float4 x = rd_load4(a + (size_t)min(m0 + r, M - 1) * lda + k);
         acc[r] = fmaf(x.w, wv.w, fmaf(x.z, wv.z, fmaf(x.y, wv.y, fmaf(x.x, wv.x, acc[r]))));
       }
     }
@@ -180,49 +182,46 @@ extern "C" int ie_gemm_diag_rows(const void* A, int a_dtype, const void* W, int 
 // ------------------------------------------------------------------ few output columns (a router)
 // C[m, n] = sum_k A[m, k] W[n, k] for N of a few dozen: the tile kernel above would give all of it to one block
 // that walks K alone.  Here a block takes a row of A into shared memory and each of its eight warps takes outputs
-// n = warp, warp + 8, ...: the lanes stride k with four partial sums each, then a tree over the lanes.  The order is
-// fixed by (n, k) alone, so a row's result does not depend on how many rows share the launch.  float32 arithmetic.
-// Many rows: MR rows a block share each element of W that is read (one row a block read all of W for it: 2,048 rows of 17 outputs
-// over 2,048 columns were 143 MB from L2 and 31 us; RD_MEASURED with eight).
-template <typename TA, typename TW, int MR>
+// n = warp, warp + 8, ...: a lane takes four neighbouring k of every 128 with a sum for each (VEC; k = lane, lane + 32, ... where rows
+// of W do not start on four elements), then a tree over the lanes.  The order is fixed by (n, k) alone, so a row's result
+// does not depend on how many rows share the launch.  float32 arithmetic.  (2,048 rows of 17 outputs over 2,048 columns in
+// a step: with four rows a block and two outputs a warp 38 us, eight rows and one output 41 us, a row a block 21:
+// 17 outputs leave warps idle in the last round, and the more rows a block has the fewer blocks hide it.)
+template <typename TA, typename TW, bool VEC>
 __global__ void __launch_bounds__(256) gemm_rowdot_kernel(const TA* __restrict__ A, const TW* __restrict__ W,
-                                                          float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
-  extern __shared__ float a_s[];
+                                                          float* __restrict__ C, int N, int K, int lda, int ldw, int ldc) {
+  extern __shared__ __align__(16) float a_s[];
   pdl_trigger();
   pdl_wait();
-  const int m0 = blockIdx.x * MR;
-#pragma unroll
-  for (int r = 0; r < MR; ++r) {
-    const bool there = m0 + r < M;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) a_s[r * K + k] = there ? to_f32(A[(size_t)(m0 + r) * lda + k]) : 0.f;
-  }
+  const int m = blockIdx.x;
+  for (int k = threadIdx.x; k < K; k += blockDim.x) a_s[k] = to_f32(A[(size_t)m * lda + k]);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // blocks along y share a row's outputs in groups of eight (a few rows then still fill the device)
   for (int n = blockIdx.y * 8 + warp; n < N; n += 8 * gridDim.y) {
     const TW* w = W + (size_t)n * ldw;
-    float acc[MR][4] = {};
-    int k = lane;
-    for (; k + 96 < K; k += 128) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float wv = to_f32(w[k + 32 * u]);
-#pragma unroll
-        for (int r = 0; r < MR; ++r) acc[r][u] = fmaf(a_s[r * K + k + 32 * u], wv, acc[r][u]);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if (VEC) {
+#pragma unroll 4
+      for (int k = lane * 4; k < K; k += 128) {
+        const float4 wv = rd_load4(w + k), x = *reinterpret_cast<const float4*>(a_s + k);
+        acc[0] = fmaf(x.x, wv.x, acc[0]);
+        acc[1] = fmaf(x.y, wv.y, acc[1]);
+        acc[2] = fmaf(x.z, wv.z, acc[2]);
+        acc[3] = fmaf(x.w, wv.w, acc[3]);
       }
-    }
+    } else {
+      int k = lane;
+      for (; k + 96 < K; k += 128) {
 #pragma unroll
-    for (int u = 0; u < 3; ++u)
-      if (k + 32 * u < K) {
-        const float wv = to_f32(w[k + 32 * u]);
-#pragma unroll
-        for (int r = 0; r < MR; ++r) acc[r][u] = fmaf(a_s[r * K + k + 32 * u], wv, acc[r][u]);
+        for (int u = 0; u < 4; ++u) acc[u] = fmaf(a_s[k + 32 * u], to_f32(w[k + 32 * u]), acc[u]);
       }
 #pragma unroll
-    for (int r = 0; r < MR; ++r) {
-      const float total = warp_sum((acc[r][0] + acc[r][1]) + (acc[r][2] + acc[r][3]));
-      if (lane == 0 && m0 + r < M) C[(size_t)(m0 + r) * ldc + n] = total;
+      for (int u = 0; u < 3; ++u)
+        if (k + 32 * u < K) acc[u] = fmaf(a_s[k + 32 * u], to_f32(w[k + 32 * u]), acc[u]);
     }
+    const float total = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+    if (lane == 0) C[(size_t)m * ldc + n] = total;
   }
 }
 
@@ -230,25 +229,24 @@ extern "C" int ie_gemm_rowdot(const void* A, int a_dtype, const void* W, int w_d
                               int lda, int ldw, int ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return IE_OK;
   if (K <= 0 || (size_t)K * sizeof(float) > 200 * 1024) return IE_BAD_SIZE;
-  // few rows (decode tokens): a block a row and eight outputs, so that the weight rows stream through many blocks; from 512 rows
-  // on eight rows a block still fill the device
-  const bool many = M >= 512 && (size_t)K * sizeof(float) <= 12 * 1024;
-  const size_t smem = (size_t)K * sizeof(float) * (many ? 8 : 1);
-  const dim3 grid(many ? (M + 7) / 8 : M, M <= 128 ? (N + 7) / 8 : 1);
-#define RD_RUN(TA, TW, MR)                                                                                         \
+  const bool vec = K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)W & 15) == 0;
+  const size_t smem = (size_t)K * sizeof(float);
+  // few rows (decode tokens): a block a row and eight outputs, so that the weight rows stream through many blocks
+  const dim3 grid(M, M <= 128 ? (N + 7) / 8 : 1);
+#define RD_RUN(TA, TW, VEC)                                                                                        \
   {                                                                                                                \
     if (smem > 47 * 1024) {                                                                                        \
-      cudaError_t e = cudaFuncSetAttribute(gemm_rowdot_kernel<TA, TW, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+      cudaError_t e = cudaFuncSetAttribute(gemm_rowdot_kernel<TA, TW, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                            (int)smem);                                                             \
       if (e != cudaSuccess) return (int)e;                                                                         \
     }                                                                                                              \
-    return launch_k(gemm_rowdot_kernel<TA, TW, MR>, grid, 256, smem, stream, (const TA*)A, (const TW*)W, C, M, N, K, lda, \
-                    ldw, ldc);                                                                                     \
+    return launch_k(gemm_rowdot_kernel<TA, TW, VEC>, grid, 256, smem, stream, (const TA*)A, (const TW*)W, C, N, K, lda, ldw, \
+                    ldc);                                                                                          \
   }
-#define RD_GO(TA, TW)                                                                                              \
-  {                                                                                                                \
-    if (many) RD_RUN(TA, TW, 8);                                                                                   \
-    RD_RUN(TA, TW, 1);                                                                                             \
+#define RD_GO(TA, TW)             \
+  {                               \
+    if (vec) RD_RUN(TA, TW, true); \
+    RD_RUN(TA, TW, false);        \
   }
   if (a_dtype == IE_F32 && w_dtype == IE_F32) RD_GO(float, float);
   if (a_dtype == IE_F32 && w_dtype == IE_BF16) RD_GO(float, bf16);

@@ -52,7 +52,7 @@ __global__ void outnorm_accumulate_kernel(float* __restrict__ residual, const TY
 }
 
 // Rows on 16 bytes, up to 8,192 wide: a thread keeps 8 columns at a time in registers, all loads 16 bytes a lane and in flight together
-// (element by element a row is three trips to memory, one after the other: 2,048 rows of 2,048 took 20 us, ONV_MEASURED here).
+// (element by element a row is three trips to memory, one after the other: 2,048 rows of 2,048 took 17.7 us, 8.1 here; with the mixture's sum before it 26.2, 11.1 here).
 // COMBINE: the row is not there yet; it is the weighted sum of a mixture's chosen experts plus the shared expert's,
 // sum over r of weights[t, r] * y[t * top + r] (r upward) + gate[t] * shared[t], which then never goes to memory.
 __device__ __forceinline__ void on_load8(const float* p, float (&v)[8]) {
@@ -364,7 +364,7 @@ causal_conv_kernel(const TA* __restrict__ x, int x_stride, const TW* __restrict_
 
 // bfloat16 rows on 16 bytes, filters of up to four taps: a thread takes 8 channels and 8 tokens in a row and keeps the inputs of the
 // filter's length in registers, so a row is read once, 16 bytes a lane (the kernel above reads two bytes a lane and every row
-// `taps` times).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 70 us, CV_MEASURED.
+// `taps` times).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 79 us, 23 so.
 #define CV_CH 8
 #define CV_RUN 8
 template <typename TW, int TAPS>
@@ -373,9 +373,25 @@ causal_conv_vec_kernel(const bf16* __restrict__ x, int x_stride, const TW* __res
                        long long state_slot_stride, bf16* __restrict__ out, int out_stride, const int* __restrict__ q_start,
                        const int* __restrict__ slots, int channels, int activation, int write_state) {
   pdl_trigger();
-  pdl_wait();
   const int c = (blockIdx.x * 32 + threadIdx.x) * CV_CH;
   const int req = blockIdx.y;
+  // the filter does not depend on the kernel ahead: asked for before the wait, 16 bytes at a time (a thread's 8 filters lie
+  // side by side)
+  float wv[TAPS][CV_CH], b[CV_CH];
+  if (c < channels) {
+    float flat[TAPS * CV_CH];
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i) on_load8(w + (size_t)c * TAPS + i * 8, *reinterpret_cast<float (*)[8]>(flat + i * 8));
+#pragma unroll
+    for (int e = 0; e < CV_CH; ++e)
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) wv[j][e] = flat[e * TAPS + j];
+    if (bias != nullptr) on_load8(bias + c, b);
+    else
+#pragma unroll
+      for (int e = 0; e < CV_CH; ++e) b[e] = 0.f;
+  }
+  pdl_wait();
   const int q0 = q_start[req], q1 = q_start[req + 1];
   const int t_lo = q0 + blockIdx.z * CONV_CHUNK + threadIdx.y * CV_RUN, t_hi = min(q1, t_lo + CV_RUN);
   if (q0 + (int)blockIdx.z * CONV_CHUNK >= q1 && blockIdx.z > 0) return;     // a shorter request than the step's longest
@@ -399,13 +415,7 @@ causal_conv_vec_kernel(const bf16* __restrict__ x, int x_stride, const TW* __res
     }
   };
   if (live && t_lo < t_hi) {
-    float wv[TAPS][CV_CH], b[CV_CH], in[TAPS][CV_CH];
-#pragma unroll
-    for (int e = 0; e < CV_CH; ++e) {
-      b[e] = bias != nullptr ? to_f32(bias[c + e]) : 0.f;
-#pragma unroll
-      for (int j = 0; j < TAPS; ++j) wv[j][e] = to_f32(w[(size_t)(c + e) * TAPS + j]);
-    }
+    float in[TAPS][CV_CH];
     uint4 raw[KEEP + CV_RUN];
 #pragma unroll
     for (int i = 0; i < KEEP + CV_RUN; ++i) {
@@ -454,8 +464,9 @@ extern "C" int ie_causal_conv(const void* x, int x_stride, const void* w, const 
   const int chunks = (max_q_len + CONV_CHUNK - 1) / CONV_CHUNK;       // of the step's longest request
   if (chunks > 65535) return IE_BAD_SIZE;
   dim3 grid((channels + CONV_CH - 1) / CONV_CH, n_requests, chunks), block(CONV_CH, CONV_TL);
-  const bool vec = act_dtype == IE_BF16 && taps >= 2 && taps <= 4 && channels % CV_CH == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 &&
-                   state_slot_stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)state) & 15) == 0;
+  // from a run of tokens on: a step of single tokens leaves seven threads in eight of it idle (8 requests: 10.9 us, the kernel above 6.6)
+  const bool vec = act_dtype == IE_BF16 && max_q_len >= CV_RUN && taps >= 2 && taps <= 4 && channels % CV_CH == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 &&
+                   state_slot_stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)state | (uintptr_t)w | (uintptr_t)bias) & 15) == 0;
 #define CV_GO(TW, TAPS)                                                                                            \
   return launch_k(causal_conv_vec_kernel<TW, TAPS>, dim3((channels + 32 * CV_CH - 1) / (32 * CV_CH), n_requests, chunks),   \
                   dim3(32, CONV_CHUNK / CV_RUN), 0, stream, (const bf16*)x, x_stride, (const TW*)w, (const TW*)bias, \
@@ -561,11 +572,14 @@ linear_recurrence_kernel(const TA* __restrict__ u, int u_stride, const TA* __res
 // blocks, each token's exponentials in the chain).  Here a block takes 16 channels and LS_SLICES runs of LS_TOK tokens; a
 // thread forms the decays and inputs of its run, runs it from a state of zero, and the runs' (sum of log a, end state)
 // pairs are put together by a scan in shared memory; then the run goes again from the state it really starts with.
-// 2,048 tokens of 2,048 channels: LS_MEASURED.
+// 2,048 tokens of 2,048 channels: 860 us token after token, 47 so.
 #define LS_CH 16
 #define LS_SLICES 64
 #define LS_TOK 8
-#define LS_MIN_TOKENS 64      // of the longest request of a step (64 tokens of one request: LS_AT_64)
+// Tokens of the step's longest request from which runs win, for every round of blocks on the SMs (a block fills one): one request
+// of 2,048 channels takes 14.7 us token after token and 11.1 in runs at 32 tokens; 8 requests of 64 tokens (seven rounds) 29
+// and 73, and go token after token.
+#define LS_MIN_TOKENS 32
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(LS_CH * LS_SLICES)
 linear_recurrence_runs_kernel(const TA* __restrict__ u, int u_stride, const TA* __restrict__ y_pre, int y_stride,
@@ -659,8 +673,13 @@ extern "C" int ie_linear_recurrence(const void* u, int u_stride, const void* y_p
                                     cudaStream_t stream) {
   if (n_requests <= 0 || width <= 0) return IE_OK;
   dim3 grid((width + 127) / 128, n_requests), run_grid((width + LS_CH - 1) / LS_CH, n_requests);
+  static const int n_sms = [] {
+    int dev = 0, v = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? v : 1;
+  }();
+  const long long rounds = ((long long)run_grid.x * n_requests + n_sms - 1) / n_sms;
 #define LRU_GO(TA, TW)                                                                                             \
-  if (max_q_len >= LS_MIN_TOKENS)                                                                                  \
+  if (max_q_len >= LS_MIN_TOKENS * rounds)                                                                         \
     return launch_k(linear_recurrence_runs_kernel<TA, TW>, run_grid, LS_CH * LS_SLICES, 0, stream, (const TA*)u, u_stride, \
                     (const TA*)y_pre, y_stride, r_pre, i_pre, g_stride, (const TW*)r_bias, (const TW*)i_bias,       \
                     (const TW*)lam, state, (TA*)out, out_stride, q_start, slots, width, decay_scale, out_scale, write_state); \

@@ -28,7 +28,9 @@ from .linear import Linear
 from .registry import register_mixer
 
 
-CHUNK_MIN_TOKENS = 64                # longest request of a step from which chunks beat a token after another
+# longest request of a step from which chunks beat a token after another (32 heads of 64, us token after token and in chunks: one
+# request of 64 tokens 40 and 47, of 128 78 and 59; 8 requests of 64 tokens 55 and 72)
+CHUNK_MIN_TOKENS = 128
 CHUNK_MAX_SCRATCH = 1 << 28          # floats (1 GB; 20,000 tokens of 32 heads of 64 x 64): longer steps go token after token
 
 

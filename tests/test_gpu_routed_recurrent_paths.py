@@ -16,7 +16,7 @@ def i32(x):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("lens,width", [((64, 1, 7, 8, 9), 40), ((511, 512, 513), 16), ((1100, 3), 33)])
+@pytest.mark.parametrize("lens,width", [((64, 1, 7, 8, 9), 40), ((511, 512, 513), 16), ((1100, 3), 33), ((32, 31), 8)])
 def test_recurrence_in_runs_of_tokens(dtype, lens, width):
     from inf_engine_b200 import kernels as k
     N, R = sum(lens), len(lens)

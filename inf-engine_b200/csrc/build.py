@@ -34,7 +34,7 @@ BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-r
 LIBRARIES = {
     "core": ["elementwise.cu", "rowwise.cu", "sequence.cu", "routed.cu", "attention_general.cu", "gemm_simt.cu", "gemm_f32.cu",
              "sampling.cu", "headwise.cu", "gating.cu", "stream_shift.cu", "headmix.cu", "matrix_memory.cu", "stream_norm.cu",
-             "convqkv.cu"],
+             "convqkv.cu", "prenorm_layers.cu"],
 }
 HEADERS = ["common.cuh"]
 

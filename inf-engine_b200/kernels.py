@@ -91,6 +91,10 @@ def core():
         lib.ie_headnorm_kv_write.argtypes = [P, P, P, I, I, I, P, P, I, F, P, P, P, I, I, I, I, I, I, I, I, P]
         lib.ie_gemm_simt.argtypes = [P, I, P, I, P, I, I, I, I, I, I, I, P]
         lib.ie_gemm_simt_batched.argtypes = [P, I, P, I, P, I, I, I, I, I, I, I, I, L, L, L, P]
+        lib.ie_prenorm_layers_sizes.argtypes = [P, P]
+        lib.ie_prenorm_layers_sizes.restype = c_int
+        lib.ie_prenorm_layers.argtypes = [P, I, P, P, P]
+        lib.ie_prenorm_layers.restype = c_int
         lib.ie_gemm_diag_rows.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P]
         lib.ie_gemm_diag_rows.restype = c_int
         lib.ie_gemm_rowdot.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P]
@@ -152,6 +156,16 @@ def core():
         _core = lib
         _apply_check_limits()
     return _core
+
+
+def prenorm_layers(layers: int, n_layers: int, step: int) -> None:
+    """The launches of a step through ``n_layers`` plain pre-norm layers; ``layers`` and ``step`` are the addresses of the
+    structures of ``csrc/prenorm_layers.cu`` (``parts/prenorm_layers.py`` fills them)."""
+    global LAUNCHES
+    count = c_int()
+    rc = core().ie_prenorm_layers(layers, n_layers, step, ctypes.addressof(count), _stream())
+    LAUNCHES += count.value - 1
+    _check(rc, "prenorm_layers")
 
 
 # ------------------------------------------------------------------ elementwise

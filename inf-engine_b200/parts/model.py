@@ -13,6 +13,7 @@ from ..cache.manager import CacheManager, CacheRequirement
 from .attention import CacheView
 from .linear import Linear, stream_normed
 from .norms import add_pending
+from .prenorm_layers import NativeLayers
 from ..weights.loader import ExpectedTensor
 from .registry import block_class, build_block, build_norm, norm_class, register_model
 
@@ -46,6 +47,7 @@ class DecoderModel:
         # a decode step is captured as a graph only if every block that runs says it may be
         self.graph_safe = all(getattr(self.layers[e.layer], "graph_safe", False) for e in spec.schedule)
         self._views: list[CacheView] | None = None
+        self._native: NativeLayers | None = None     # all layers of a step with prompt portions in one native call
 
     # ------------------------------------------------------------------ cache
     def cache_requirements(self) -> list[CacheRequirement]:
@@ -77,6 +79,8 @@ class DecoderModel:
             src = i if e.cache_from is None else e.cache_from
             views.append(view(manager.bindings[src], e.cache_from is None))
         self._views = views
+        between = type(self).before_entry is not DecoderModel.before_entry     # something happens to the stream between layers
+        self._native = None if between else NativeLayers.of(self, views)
 
     # ---------------------------------------------------------------- forward
     def embed(self, ctx) -> torch.Tensor:
@@ -110,7 +114,10 @@ class DecoderModel:
         ctx.handover = None
         ctx.residual_cast = None
         last = len(spec.schedule) - 1
-        for i, e in enumerate(spec.schedule):
+        native = self._native is not None and self._native.takes(ctx)
+        if native:
+            residual, pending = self._native.forward(residual, pending, ctx)
+        for i, e in enumerate(() if native else spec.schedule):
             # the norm that the residual meets after this block: the next block's first, or the final one
             nxt = self.layers[spec.schedule[i + 1].layer] if i < last else None
             ctx.norm_after_block = getattr(nxt, "mixer_norm", None) if nxt is not None else self.final_norm

@@ -271,8 +271,8 @@ __global__ void __launch_bounds__(GD_THREADS) gated_delta_kernel(GatedDeltaParam
 //   finish   (block: chunk, head): the outputs, their norm and gate
 // All of it float32 products and sums; exponents are sums of log g, so a decay close to one keeps its digits
 // (S + expm1(L_end) S).  Tokens beyond the request's last have beta = 0, log g = 0 and zero vectors.
-// 2,048 tokens of 32 heads of 64: 1,221 us alone and 1,713 in a step token after token, 328 so
-// (120 prepare, 120 carry, 69 finish).
+// 2,048 tokens of 32 heads of 64: 1,221 us alone and 1,713 in a step token after token, 293 so
+// (120 prepare, 85 carry, 69 finish).
 #define GD_C 64
 #define GD_CHUNKED (GD_DK % 16 == 0 && GD_DV % 16 == 0 && GD_DK >= 32 && GD_DK <= 128 && GD_DV >= 32 && GD_DV <= 128)
 #if GD_CHUNKED
@@ -454,11 +454,15 @@ __device__ __forceinline__ void gd_copy16(float* dst, const float* src) {
 constexpr int GD_SLICE = 16;                      // value channels of a carry block
 constexpr int GD_CARRY_STAGE = GD_C * GD_PK + GD_DK * GD_PC + GD_SLICE * GD_PC;
 
-// 256 threads: four groups of 64 take a quarter of the inner length each (4 x 4 outputs a thread, 64 x 16 a group and pass)
-__global__ void __launch_bounds__(GD_CT) gated_delta_carry_kernel(GatedDeltaChunks d) {
+// Groups of 64 threads take an equal part of the inner length each (4 x 4 outputs a thread, 64 x 16 a group and pass).  A chunk is a
+// chain of two short products and four barriers, so eight groups where DK allows (2,048 tokens of 32 heads: four groups 328 us
+// for the three kernels, eight 293).
+constexpr int GD_GROUPS = GD_DK % 32 == 0 ? 8 : 4;
+constexpr int GD_CARRY_T = 64 * GD_GROUPS;
+__global__ void __launch_bounds__(GD_CARRY_T) gated_delta_carry_kernel(GatedDeltaChunks d) {
   extern __shared__ __align__(16) float gd_smem[];
   float* const st = gd_smem + 2 * GD_CARRY_STAGE;             // [GD_SLICE][GD_PK] the state's columns
-  float* const red = st + GD_SLICE * GD_PK;                   // [4][64][GD_SLICE + 1]
+  float* const red = st + GD_SLICE * GD_PK;                   // [GD_GROUPS][64][GD_SLICE + 1]
   const GatedDeltaParams& p = d.p;
   pdl_trigger();
   pdl_wait();
@@ -476,17 +480,17 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_carry_kernel(GatedDeltaChun
       float* const w = gd_smem + (c & 1) * GD_CARRY_STAGE;
       float* const kd = w + GD_C * GD_PK;
       float* const u = kd + GD_DK * GD_PC;
-      for (int i = tid; i < GD_C * GD_DK / 4; i += GD_CT) {
+      for (int i = tid; i < GD_C * GD_DK / 4; i += GD_CARRY_T) {
         gd_copy16(w + (i / (GD_DK / 4)) * GD_PK + (i % (GD_DK / 4)) * 4, d.w + slot * (GD_C * GD_DK) + i * 4);
         gd_copy16(kd + (i / (GD_C / 4)) * GD_PC + (i % (GD_C / 4)) * 4, d.kd + slot * (GD_C * GD_DK) + i * 4);
       }
-      for (int i = tid; i < GD_SLICE * GD_C / 4; i += GD_CT)
+      for (int i = tid; i < GD_SLICE * GD_C / 4; i += GD_CARRY_T)
         gd_copy16(u + (i / (GD_C / 4)) * GD_PC + (i % (GD_C / 4)) * 4, d.u + slot * (GD_C * GD_DV) + j0 * GD_C + i * 4);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(0);
-  for (int i = tid; i < GD_DK * GD_SLICE; i += GD_CT)
+  for (int i = tid; i < GD_DK * GD_SLICE; i += GD_CARRY_T)
     st[(i % GD_SLICE) * GD_PK + i / GD_SLICE] = state[(size_t)(i / GD_SLICE) * GD_DV + i % GD_SLICE];
   const int group = tid >> 6, r = (tid & 63) >> 2, jc = tid & 3;
   auto leave = [&](float (&acc)[4][4]) {
@@ -495,10 +499,12 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_carry_kernel(GatedDeltaChun
 #pragma unroll
       for (int j = 0; j < 4; ++j) red[(group * 64 + r + 16 * i) * (GD_SLICE + 1) + jc + 4 * j] = acc[i][j];
   };
-  auto sum4 = [&](int row, int j) {
+  auto total = [&](int row, int j) {
     const float* at = red + row * (GD_SLICE + 1) + j;
     constexpr int step = 64 * (GD_SLICE + 1);
-    return (at[0] + at[step]) + (at[2 * step] + at[3 * step]);
+    float v = (at[0] + at[step]) + (at[2 * step] + at[3 * step]);
+    if (GD_GROUPS == 8) v += (at[4 * step] + at[5 * step]) + (at[6 * step] + at[7 * step]);
+    return v;
   };
   for (int c = 0; c < chunks; ++c) {
     const size_t slot = gd_chunk(q0, req, c, h, p.n_heads);
@@ -510,17 +516,17 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_carry_kernel(GatedDeltaChun
     fetch(c + 1);
     const float grow = expm1f(d.tok[slot * GD_TOK + GD_C]);
     // the start state, for the outputs
-    for (int i = tid; i < GD_SLICE * GD_DK; i += GD_CT)
+    for (int i = tid; i < GD_SLICE * GD_DK; i += GD_CARRY_T)
       d.s0[slot * (GD_DK * GD_DV) + j0 * GD_DK + i] = st[(i / GD_DK) * GD_PK + i % GD_DK];
     {
       float acc[4][4] = {};
-      gd_product<4, 4>(acc, w + r * GD_PK, GD_PK, st + jc * GD_PK, GD_PK, group * (GD_DK / 4), (group + 1) * (GD_DK / 4), 16, 4);
+      gd_product<4, 4>(acc, w + r * GD_PK, GD_PK, st + jc * GD_PK, GD_PK, group * (GD_DK / GD_GROUPS), (group + 1) * (GD_DK / GD_GROUPS), 16, 4);
       leave(acc);
     }
     __syncthreads();
-    for (int i = tid; i < GD_SLICE * GD_C; i += GD_CT) {
+    for (int i = tid; i < GD_SLICE * GD_C; i += GD_CARRY_T) {
       const int j = i / GD_C, t = i % GD_C;
-      const float v = u[j * GD_PC + t] - sum4(t, j);
+      const float v = u[j * GD_PC + t] - total(t, j);
       u[j * GD_PC + t] = v;
       d.u[slot * (GD_C * GD_DV) + j0 * GD_C + i] = v;
     }
@@ -529,21 +535,21 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_carry_kernel(GatedDeltaChun
     for (int i0 = 0; i0 < GD_DK; i0 += 64) {
       float acc[4][4] = {};
       // rows beyond DK (a size that 64 does not divide) read the rows that follow in shared memory and are dropped below
-      gd_product<4, 4>(acc, kd + (i0 + r) * GD_PC, GD_PC, u + jc * GD_PC, GD_PC, group * (GD_C / 4), (group + 1) * (GD_C / 4), 16, 4);
+      gd_product<4, 4>(acc, kd + (i0 + r) * GD_PC, GD_PC, u + jc * GD_PC, GD_PC, group * (GD_C / GD_GROUPS), (group + 1) * (GD_C / GD_GROUPS), 16, 4);
       leave(acc);
       __syncthreads();
-      for (int i = tid; i < GD_SLICE * 64; i += GD_CT) {
+      for (int i = tid; i < GD_SLICE * 64; i += GD_CARRY_T) {
         const int j = i / 64, row = i % 64;
         if (i0 + row < GD_DK) {
           float* at = st + j * GD_PK + i0 + row;
-          *at = fmaf(grow, *at, *at) + sum4(row, j);
+          *at = fmaf(grow, *at, *at) + total(row, j);
         }
       }
       __syncthreads();
     }
   }
   if (p.write_state)
-    for (int i = tid; i < GD_DK * GD_SLICE; i += GD_CT)
+    for (int i = tid; i < GD_DK * GD_SLICE; i += GD_CARRY_T)
       state[(size_t)(i / GD_SLICE) * GD_DV + i % GD_SLICE] = st[(i % GD_SLICE) * GD_PK + i / GD_SLICE];
 }
 
@@ -618,7 +624,7 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_finish_kernel(GatedDeltaChu
 
 constexpr size_t GD_SLOT_FLOATS = (size_t)2 * GD_C * GD_DK + GD_C * GD_DV + GD_C * GD_C + GD_DK * GD_DV + GD_TOK;
 constexpr size_t GD_PREPARE_SMEM = (size_t)(2 * GD_C * GD_PK + GD_C * GD_PC) * 4;
-constexpr size_t GD_CARRY_SMEM = (size_t)(2 * GD_CARRY_STAGE + GD_SLICE * GD_PK + 4 * 64 * (GD_SLICE + 1)) * 4;
+constexpr size_t GD_CARRY_SMEM = (size_t)(2 * GD_CARRY_STAGE + GD_SLICE * GD_PK + GD_GROUPS * 64 * (GD_SLICE + 1)) * 4;
 constexpr size_t GD_FINISH_SMEM = (size_t)(GD_C * GD_PK + GD_DV * GD_PK + GD_C * GD_PC + GD_DV * GD_PC) * 4;
 
 template <typename TA, typename TW>
@@ -634,7 +640,7 @@ static int gd_launch_chunks(const GatedDeltaChunks& d, int n_requests, int chunk
   if (ready != cudaSuccess) return (int)ready;
   const dim3 grid(chunks, d.p.n_heads, n_requests);
   int rc = launch_k(gated_delta_prepare_kernel<TA, TW>, grid, GD_CT, GD_PREPARE_SMEM, stream, d);
-  if (!rc) rc = launch_k(gated_delta_carry_kernel, dim3(GD_DV / GD_SLICE, d.p.n_heads, n_requests), GD_CT, GD_CARRY_SMEM, stream, d);
+  if (!rc) rc = launch_k(gated_delta_carry_kernel, dim3(GD_DV / GD_SLICE, d.p.n_heads, n_requests), GD_CARRY_T, GD_CARRY_SMEM, stream, d);
   if (!rc) rc = launch_k(gated_delta_finish_kernel<TA, TW>, grid, GD_CT, GD_FINISH_SMEM, stream, d);
   return rc;
 }

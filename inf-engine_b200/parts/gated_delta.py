@@ -28,9 +28,10 @@ from .linear import Linear
 from .registry import register_mixer
 
 
-# longest request of a step from which chunks beat a token after another (32 heads of 64, us token after token and in chunks: one
-# request of 64 tokens 40 and 47, of 128 78 and 59; 8 requests of 64 tokens 55 and 72)
-CHUNK_MIN_TOKENS = 128
+# When chunks beat a token after another, in us of heads of 64 x 64 (measured): the chain takes 0.6 a token of the longest request, the
+# chunks 40 and 0.25 for each chunk of 64 tokens and head of all requests.  One request of 32 heads from about 85 tokens on
+# (128 tokens: 80 and 56, 2,048: 1,228 and 293); 8 requests of 128 tokens stay a chain (108, in chunks 148).
+CHAIN_US_PER_TOKEN, CHUNKS_US, CHUNKS_US_PER_TOKEN_AND_HEAD = 0.6, 40.0, 0.25 / 64
 CHUNK_MAX_SCRATCH = 1 << 28          # floats (1 GB; 20,000 tokens of 32 heads of 64 x 64): longer steps go token after token
 
 
@@ -112,7 +113,7 @@ class GatedDeltaMixer:
         a_pre = proj[:, c0 + self.vw + s.n_heads:]
         mixed = rt.ws.take("gated_delta_mixed", (n, self.vw), rt.act_dtype)
         scratch = None
-        if ctx.max_q_len >= CHUNK_MIN_TOKENS:
+        if CHUNKS_US + CHUNKS_US_PER_TOKEN_AND_HEAD * s.n_heads * n < CHAIN_US_PER_TOKEN * ctx.max_q_len:
             floats = kernels.gated_delta_scratch_floats(n, ctx.n_requests, s.n_heads, s.head_dim, s.v_head_dim)
             if 0 < floats <= CHUNK_MAX_SCRATCH:
                 scratch = rt.ws.take("gated_delta_chunks", (floats,), torch.float32)

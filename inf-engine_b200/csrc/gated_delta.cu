@@ -601,8 +601,8 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_finish_kernel(GatedDeltaChu
   gd_product<4, TN>(acc, qs + r * GD_PK, GD_PK, s0 + cc * GD_PK, GD_PK, 0, GD_DK);
   gd_product<4, TN>(acc, qk + r * GD_PC, GD_PC, u + cc * GD_PC, GD_PC, 0, GD_C);
   __syncthreads();
-  float* const so = gd_smem;                      // [GD_C][GD_DV + 1], where qs and s0 were
-  static_assert(GD_C * (GD_DV + 1) <= GD_C * GD_PK + GD_DV * GD_PK, "the outputs take the place of the first operands");
+  float* const so = gd_smem;                      // [GD_C][GD_DV + 1], where the operands were (both products have read them)
+  static_assert(GD_C * (GD_DV + 1) <= (GD_C + GD_DV) * (GD_PK + GD_PC), "the outputs take the place of the operands");
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll

@@ -1,5 +1,6 @@
 """The gated delta rule in chunks of 64 tokens against float64, token after token: lengths around a chunk's edges, several
-requests, a padding row without a slot, a state that is only read; its error beside the token-by-token kernel's."""
+requests, a padding row without a slot, a state that is only read; its error beside the token-by-token kernel's.  Key sizes of
+every kind: eight and four groups of threads, a last pass over the rows of the state that is part empty, one pass and two."""
 import pytest
 import torch
 
@@ -23,7 +24,9 @@ def plain(q, k, v, b, a, gate, a_log, dt_bias, gain, S, G):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("dk,dv,H,G,lens", [(64, 64, 4, 2, (1, 64, 65, 7, 200)), (64, 128, 2, 1, (63, 130)), (128, 128, 2, 2, (129, 2))])
+@pytest.mark.parametrize("dk,dv,H,G,lens", [(64, 64, 4, 2, (1, 64, 65, 7, 200)), (64, 128, 2, 1, (63, 130)), (128, 128, 2, 2, (129, 2)),
+                                             (32, 128, 4, 2, (130, 3)), (48, 48, 2, 1, (66, 2)), (80, 32, 3, 3, (129, 5)),
+                                             (96, 96, 2, 1, (70, 64))])
 def test_chunks_against_the_recurrence(dtype, dk, dv, H, G, lens):
     from inf_engine_b200 import kernels
     g = torch.Generator("cuda").manual_seed(sum(lens) + dk)

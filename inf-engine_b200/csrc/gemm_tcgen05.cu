@@ -55,7 +55,7 @@ struct TcParams {
   const int* tiles;
   const int* place;
   int max_tiles;
-  // block-diagonal form: output columns in groups of diag_n, group b reads columns b K .. of A (0: every column reads all of A)
+  // block-diagonal form: output columns in groups of diag_n, group b reads columns b K .. of A
   int diag_n;
 };
 
@@ -270,7 +270,12 @@ __device__ __forceinline__ void tc_flush(const TcParams& p, const unsigned char*
   }
 }
 
-template <int BN, bool GROUPED>
+// DIAG: the block-diagonal form, float32 result.  Every 64 k make an accumulator of their own, and the epilogue adds them up in
+// registers, k upward.  The tensor cores cut bits off at every step of 16 k that they add: one chain over K has 2.1 times the
+// error of float32 multiply-adds at K of 256 and 2.9 times at 512 (and these sums drive a recurrence); sums of 64 have
+// 0.97 of it at 128, 0.72 at 256 and 0.53 at 512.  2,048 rows of 8 blocks of 256 x 256: 90 us on CUDA cores, 9.2 as one chain,
+// 11.4 so.
+template <int BN, bool GROUPED, bool DIAG>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                      const __grid_constant__ CUtensorMap map_w,
                                                                      TcParams p) {
@@ -325,7 +330,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
         const int mt = t % m_tiles, n0 = (t / m_tiles) * BN;
         const int m0 = GROUPED ? p.tiles[4 * mt + 1] : mt * BM;
         const int w0 = GROUPED ? p.tiles[4 * mt] * p.N + n0 : n0;      // the expert's own rows of the stacked weights
-        const int a_k0 = (!GROUPED && p.diag_n) ? (n0 / p.diag_n) * p.K : 0;
+        const int a_k0 = DIAG ? (n0 / p.diag_n) * p.K : 0;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (failed || !tc_mbar_wait(empty0 + 8 * s, phase ^ 1)) { atomicExch(&g_tc_error, 1); failed = 1; break; }
           const uint32_t bar = full0 + 8 * s;
@@ -343,15 +348,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
       const uint32_t idesc = umma_idesc(BM, BN);
       int s = 0;
       uint32_t phase = 0;
-      int it = 0;
-      for (int t = blockIdx.x; t < total_tiles && !failed; t += gridDim.x, ++it) {
+      int it = 0, part = 0;
+      const int parts = DIAG ? k_blocks : 1, part_blocks = DIAG ? 1 : k_blocks;      // accumulators of a tile, stages in each
+      for (int t = blockIdx.x; t < total_tiles && !failed; ++it) {
         const int buf = it & 1;
         const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
         // the epilogue has drained this accumulator (immediately true the first time round)
         if (!tc_mbar_wait(acc_empty0 + 8 * buf, acc_phase ^ 1)) { atomicExch(&g_tc_error, 4); failed = 1; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        for (int kb = 0; kb < part_blocks; ++kb) {
           if (failed || !tc_mbar_wait(full0 + 8 * s, phase)) { atomicExch(&g_tc_error, 2); failed = 1; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_src = ring + s * STAGE_BYTES, w_src = a_src + A_BYTES;
@@ -365,6 +371,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
         }
         if (failed) break;
         umma_commit(acc_full0 + 8 * buf);       // arrives when the whole accumulator is final
+        if (++part == parts) { part = 0; t += gridDim.x; }
       }
     }
   } else {
@@ -373,7 +380,51 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
     unsigned char* stage = smem_raw + (ring - saddr(smem_raw)) + (size_t)p.n_stages * STAGE_BYTES + (warp - 2) * TC_STAGE_BYTES;
     const int out32 = tc_out_bytes32(p.epi);
     int it = 0;
-    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+    bool ok = true;
+    for (int t = blockIdx.x; DIAG && t < total_tiles && ok; t += gridDim.x) {
+      const int m = (t % m_tiles) * BM + quarter * 32 + lane, n0 = (t / m_tiles) * BN;
+      float sum[BN / 32][32];
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[c][j] = 0.f;
+#pragma unroll 1
+      for (int part = 0; part < k_blocks && ok; ++part, ++it) {
+        const int buf = it & 1;
+        ok = !failed && tc_mbar_wait(acc_full0 + 8 * buf, (uint32_t)(it >> 1) & 1u);
+        if (!ok && lane == 0) { atomicExch(&g_tc_error, 3); failed = 1; }
+        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0 && !failed;
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + 32 * c), r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[c][j] += __uint_as_float(r[j]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * buf) : "memory");
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) {
+        uint32_t r[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[c][j]);
+        if (p.staged) {
+          tc_stage_row(p, stage, lane, 0, TC_EPI_F32, r);
+          __syncwarp();
+          tc_flush<false>(p, stage, lane, m - lane, m, (size_t)(n0 + 32 * c) * 4);
+          __syncwarp();
+        } else {
+          tc_epilogue_store(p, m, n0 + 32 * c, r);
+        }
+      }
+    }
+    for (int t = blockIdx.x; !DIAG && t < total_tiles; t += gridDim.x, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
       const int mt = t % m_tiles, n0 = (t / m_tiles) * BN;
@@ -382,7 +433,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
         const int r = quarter * 32 + lane, src = p.tiles[4 * mt + 1] + r;
         m = r < p.tiles[4 * mt + 2] ? (p.place != nullptr ? p.place[src] : src) : -1;
       }
-      bool ok = !failed && tc_mbar_wait(acc_full0 + 8 * buf, acc_phase);
+      ok = !failed && tc_mbar_wait(acc_full0 + 8 * buf, acc_phase);
       if (!ok && lane == 0) { atomicExch(&g_tc_error, 3); failed = 1; }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0 && !failed;
       if (!ok) break;
@@ -454,7 +505,7 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int cols, int 
   return r == CUDA_SUCCESS ? IE_OK : IE_BAD_ALIGN;
 }
 
-template <int BN, bool GROUPED>
+template <int BN, bool GROUPED, bool DIAG = false>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, TcParams p, int n_sms, cudaStream_t stream) {
   const uint32_t stage = (BM + BN) * BK * 2;
   int n_stages = (200 * 1024 - 1024) / stage;
@@ -463,13 +514,13 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, TcParams p, i
   const size_t smem = (size_t)n_stages * stage + 1024 + 4 * TC_STAGE_BYTES;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, GROUPED, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
   const int tiles = (GROUPED ? p.max_tiles : (p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   const int grid = tiles < n_sms ? tiles : n_sms;
-  return launch_k(gemm_tcgen05_kernel<BN, GROUPED>, grid, TC_THREADS, smem, stream, ma, mw, p);
+  return launch_k(gemm_tcgen05_kernel<BN, GROUPED, DIAG>, grid, TC_THREADS, smem, stream, ma, mw, p);
 }
 
 }  // namespace
@@ -553,16 +604,15 @@ extern "C" int ie_gemm_tcgen05_diag(const void* A, const void* W, float* C, int 
   if ((long long)blocks * n > 0x7fffffffLL || (long long)blocks * K > 0x7fffffffLL) return IE_BAD_SIZE;
   if (!ie_gemm_tcgen05_supports(M, n, K, lda, K)) return IE_BAD_SIZE;
   if (((uintptr_t)A | (uintptr_t)W) & 15) return IE_BAD_ALIGN;
-  const int bn = n % 256 == 0 ? 256 : 128;
   CUtensorMap ma, mw;
   int rc = make_map(&ma, A, M, blocks * K, lda, BM);
   if (rc) return rc;
-  rc = make_map(&mw, W, blocks * n, K, K, bn);
+  rc = make_map(&mw, W, blocks * n, K, K, 128);
   if (rc) return rc;
   TcParams p = {};
   p.C = C; p.M = M; p.N = blocks * n; p.K = K; p.ldc = ldc; p.epi = TC_EPI_F32; p.diag_n = n;
   p.staged = (((uintptr_t)C & 15) == 0 && ldc % 4 == 0) ? 1 : 0;
-  return bn == 256 ? launch_tc<256, false>(ma, mw, p, n_sms, stream) : launch_tc<128, false>(ma, mw, p, n_sms, stream);
+  return launch_tc<128, false, true>(ma, mw, p, n_sms, stream);
 }
 
 extern "C" int ie_gemm_tcgen05(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc,

@@ -436,8 +436,9 @@ DIAG_FEW_ROWS = 16      # up to here a warp an output column beats tiles of 64 r
 
 def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     """``gemm_simt_batched`` by the kernel that suits the rows: a warp an output for a few, the tcgen05 tensor cores for
-    bfloat16 operands from a tile of 128 rows on (their products are exact in float32, the sums float32), tiles on CUDA
-    cores else."""
+    bfloat16 operands from a tile of 128 rows on, tiles on CUDA cores else.  On the tensor cores products
+    are exact in float32 and the sums, float32 too, are taken over 64 k at a time, so that they are no further off than
+    multiply-adds; a product of 64 k in all would be."""
     blocks, n, k = w.shape
     m = a.shape[0]
     assert a.shape[1] == blocks * k and out.shape == (m, blocks * n) and out.dtype is torch.float32
@@ -446,7 +447,7 @@ def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     if m <= DIAG_FEW_ROWS and k % 4 == 0 and a.stride(0) % 4 == 0 and aligned:
         _check(core().ie_gemm_diag_rows(_ptr(a), dtype_code(a.dtype), _ptr(w), dtype_code(w.dtype), _ptr(out), m, blocks, n, k,
                                         a.stride(0), out.stride(0), _stream()), f"gemm_diag_rows(blocks={blocks}, n={n}, k={k})")
-    elif (m >= 128 and a.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and n % 128 == 0 and aligned
+    elif (m >= 128 and k >= 128 and a.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and n % 128 == 0 and aligned
           and gemm_tcgen05_supports(m, n, k, a.stride(0), k)):
         _check(tcgen05_library().ie_gemm_tcgen05_diag(_ptr(a), _ptr(w), _ptr(out), m, blocks, n, k, a.stride(0), out.stride(0),
                                                       sm_count(), _stream()), f"gemm_tcgen05_diag(blocks={blocks}, n={n}, k={k})")

@@ -16,8 +16,9 @@
 // registers while the tile before is being run: (A) they go to shared memory as float32, a thread per token forms
 // beta and g and a warp per token makes q and k unit vectors;
 // (B) every thread runs the tile's tokens in order; (C) a warp per token norms and gates the outputs.  The order
-// of every sum is fixed by the token and the channel alone, so a token's result does not depend on how the
-// sequence was cut into steps or on what else the step holds.  A decode step is a tile of one token.
+// of every sum is fixed by the token and the channel alone, so this kernel's result does not depend on how the
+// sequence was cut into steps or on what else the step holds.  A decode step is a tile of one token.  (The chunked form
+// below sums in another order; the 32-bit path never takes it.)
 #include "common.cuh"
 
 #if !defined(IE_GD_DK) || !defined(IE_GD_DV)

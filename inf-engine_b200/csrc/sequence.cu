@@ -502,8 +502,9 @@ extern "C" int ie_causal_conv(const void* x, int x_stride, const void* w, const 
 // 1 - a^2 is formed as -expm1(2 log a), which keeps its digits when a is close to one; and while a is above one
 // half the state is moved by S += (a - 1) S + input with a - 1 = expm1(log a): a float32 a = 1 - 2.5e-6 is off by up
 // to a hundredth of its distance from one, which over a thousand tokens shows in the fifth digit of S.  A thread owns a channel
-// of a request and walks the step's tokens in order; the loads of a token do not depend on S, so several
-// tokens' loads are in flight while the chain runs.
+// of a request and walks the step's tokens in order, so that a cut of the sequence changes nothing; the loads of a token do not
+// depend on S, so several tokens' loads are in flight while the chain runs.  (The form for many tokens, below, sums in another
+// order; the 32-bit path never takes it.)
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float gelu_tanh_f(float z) {

@@ -435,7 +435,8 @@ DIAG_FEW_ROWS = 16      # up to here a warp an output column beats tiles of 64 r
 
 
 def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """``gemm_simt_batched`` by the kernel that suits the rows: a warp an output for a few, the tcgen05 tensor cores for
+    """``gemm_simt_batched`` by the kernel that suits the rows.  float32 rows (the 32-bit path): always that kernel, whose order of
+    sums does not depend on how many rows share the launch.  bfloat16 rows: a warp an output for a few, the tcgen05 tensor cores for
     bfloat16 operands from a tile of 128 rows on, tiles on CUDA cores else.  On the tensor cores products
     are exact in float32 and the sums, float32 too, are taken over 64 k at a time, so that they are no further off than
     multiply-adds; a product of 64 k in all would be."""
@@ -444,7 +445,8 @@ def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     assert a.shape[1] == blocks * k and out.shape == (m, blocks * n) and out.dtype is torch.float32
     assert a.stride(1) == 1 and w.is_contiguous() and out.stride(1) == 1
     aligned = a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-    if m <= DIAG_FEW_ROWS and k % 4 == 0 and a.stride(0) % 4 == 0 and aligned:
+    few = a.dtype is torch.bfloat16 and m <= DIAG_FEW_ROWS
+    if few and k % 4 == 0 and a.stride(0) % 4 == 0 and aligned:
         _check(core().ie_gemm_diag_rows(_ptr(a), dtype_code(a.dtype), _ptr(w), dtype_code(w.dtype), _ptr(out), m, blocks, n, k,
                                         a.stride(0), out.stride(0), _stream()), f"gemm_diag_rows(blocks={blocks}, n={n}, k={k})")
     elif (m >= 128 and k >= 128 and a.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and n % 128 == 0 and aligned

@@ -13,8 +13,10 @@ With x the mixer's input, per token:
 then ``o`` is divided by its root mean square over the head, multiplied by a gain of the head's size and by
 ``silu(gate)``, and projected back by ``o_proj``.  The projections and the convolutions are in the activation
 type; everything from there to the gated output is float32 inside one kernel (``csrc/gated_delta.cu``), which runs
-a step's tokens of every request in order from the state the step before left: a whole prompt, a portion and a
-single decoded token take the same path.
+a step's tokens of every request from the state the step before left.  On the 32-bit path they go one after another: a
+whole prompt, a portion and a single decoded token take the same path and give the same bits, whatever else the step holds.  In
+bfloat16 steps of long enough requests go in chunks of tokens, which sum in another order: the same float32 arithmetic, but
+a token's result then depends, by rounding, on the cut and on the step's other requests.
 """
 
 from __future__ import annotations
@@ -113,7 +115,7 @@ class GatedDeltaMixer:
         a_pre = proj[:, c0 + self.vw + s.n_heads:]
         mixed = rt.ws.take("gated_delta_mixed", (n, self.vw), rt.act_dtype)
         scratch = None
-        if CHUNKS_US + CHUNKS_US_PER_TOKEN_AND_HEAD * s.n_heads * n < CHAIN_US_PER_TOKEN * ctx.max_q_len:
+        if not rt.exact and CHUNKS_US + CHUNKS_US_PER_TOKEN_AND_HEAD * s.n_heads * n < CHAIN_US_PER_TOKEN * ctx.max_q_len:
             floats = kernels.gated_delta_scratch_floats(n, ctx.n_requests, s.n_heads, s.head_dim, s.v_head_dim)
             if 0 < floats <= CHUNK_MAX_SCRATCH:
                 scratch = rt.ws.take("gated_delta_chunks", (floats,), torch.float32)

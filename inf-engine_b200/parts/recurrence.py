@@ -9,7 +9,9 @@
     S <- a S + sqrt(1 - a^2) (i * u);   out = o_proj (S * y)  S: float32, one vector a request, zero at the start
 
 The gates, the decay, the state and the product with y are float32 (``csrc/sequence.cu``); the step's tokens of
-every request run in order from the state that the step before left.
+every request start from the state that the step before left.  On the 32-bit path every sum has one order, whatever the
+step holds and however a sequence was cut.  In bfloat16 the gate products (by the step's rows) and the recurrence (runs of
+tokens side by side where the step's requests make them faster) choose between forms whose results differ by float32 rounding.
 
 ``ParallelMixer`` runs several mixers on the same input and adds what they return; each branch carries its weight
 in the sum as its own ``out_scale``.  When every branch ends in an output projection (``forward_core`` returns what
@@ -92,7 +94,7 @@ class GatedLinearRecurrence:
         kernels.block_diagonal(u, self.i_gate, gates[:, w:])
         kernels.linear_recurrence(u, proj[:, :w], gates[:, :w], gates[:, w:], self.a_bias, self.i_bias, self.lam,
                                   state.state, out, ctx.q_start, ctx.slots, ctx.n_requests, s.decay_scale, s.out_scale,
-                                  write_state=cache.write, max_q_len=ctx.max_q_len)
+                                  write_state=cache.write, max_q_len=0 if rt.exact else ctx.max_q_len)
 
     def forward(self, x: torch.Tensor, ctx, cache) -> torch.Tensor:
         rt = self.rt

@@ -295,6 +295,7 @@ constexpr int GD_PK = GD_DK + 4, GD_PC = GD_C + 4;   // row pitches in shared me
 __device__ __forceinline__ size_t gd_chunk(int q0, int req, int c, int h, int heads) {
   return (size_t)(q0 / GD_C + req + c) * heads + h;
 }
+constexpr float GD_LOG_FLOOR = -1e4f;
 __device__ __forceinline__ float gd_log_decay(float rate, float a) { return rate * (a > 20.f ? a : log1pf(expf(a))); }
 
 // acc[i][j] += sum over x of a[(r + 16 i)][x] b[(c + 16 j)][x], x in [x0, x1) (multiples of 4); four sums a thread run in order
@@ -352,7 +353,9 @@ __global__ void __launch_bounds__(GD_CT, 2) gated_delta_prepare_kernel(GatedDelt
       double lg = 0.;
       float beta = 0.f;
       if (t < nt) {
-        lg = gd_log_decay(rate, to_f32(((const TA*)p.a_pre)[(size_t)(t0 + t) * p.ba_stride + h]) + dt_bias);
+        const float log_g = gd_log_decay(rate, to_f32(((const TA*)p.a_pre)[(size_t)(t0 + t) * p.ba_stride + h]) + dt_bias);
+        // a log decay that overflowed would make differences of the sums NaN; from -104 down every exp is zero all the same
+        lg = log_g < GD_LOG_FLOOR ? GD_LOG_FLOOR : log_g;
         beta = 1.f / (1.f + expf(-to_f32(((const TA*)p.b_pre)[(size_t)(t0 + t) * p.ba_stride + h])));
       }
 #pragma unroll

@@ -71,3 +71,38 @@ def test_chunks_against_the_recurrence(dtype, dk, dv, H, G, lens):
     assert err(out, other.double()) < (3e-6 if dtype is torch.float32 else 6e-3)
     again, kept = run(torch.full((floats,), float("nan"), device="cuda"), write=False)
     assert torch.equal(again, out) and torch.equal(kept, state)
+
+
+def inputs(H, G, dk, dv, N, seed):
+    g = torch.Generator("cuda").manual_seed(seed)
+    qk, v, ba, gate = (torch.randn(N, w, device="cuda", generator=g) for w in (2 * G * dk, H * dv, 2 * H, H * dv))
+    return {"qk": qk, "v": v, "ba": ba, "gate": gate, "a_log": torch.linspace(-4, 0.5, H, device="cuda"),
+            "dt_bias": torch.linspace(-3, 1, H, device="cuda"), "gain": 1 + 0.1 * torch.randn(dv, device="cuda", generator=g),
+            "state": 0.3 * torch.randn(1, H, dk, dv, device="cuda", generator=g)}
+
+
+def both_forms(x, H, G, dk, dv):
+    """(outputs [N, H, dv], state) in chunks, and token after token"""
+    from inf_engine_b200 import kernels
+    N, got = len(x["v"]), []
+    for floats in (kernels.gated_delta_scratch_floats(N, 1, H, dk, dv), 0):
+        st, out = x["state"].clone(), torch.empty(N, H * dv, device="cuda")
+        at, slot = torch.tensor([0, N], dtype=torch.int32, device="cuda"), torch.tensor([0], dtype=torch.int32, device="cuda")
+        kernels.gated_delta(x["qk"][:, :G * dk], x["qk"][:, G * dk:], x["v"], x["ba"][:, :H], x["ba"][:, H:], x["gate"], x["a_log"],
+                            x["dt_bias"], x["gain"], st, out, at, slot, 1, H, G, dk, dv, 1e-6, 1e-5,
+                            scratch=torch.zeros(floats, device="cuda") if floats else None, max_q_len=N)
+        got.append((out.view(N, H, dv), st))
+    return got
+
+
+def test_a_decay_of_zero():
+    """A log decay that overflows to minus infinity empties the state, and both forms go on from there."""
+    H, G, dk, dv, N = 4, 2, 64, 64, 150
+    x = inputs(H, G, dk, dv, N, 5)
+    x["a_log"][1] = 100.0                         # its exp overflows: every token of the head
+    x["ba"][[0, 40, 41, 130], H + 2] = 3e38       # the product with the rate overflows: these tokens
+    (out, st), (want, want_st) = both_forms(x, H, G, dk, dv)
+    assert bool(torch.isfinite(want).all()) and bool(torch.isfinite(out).all()) and bool(torch.isfinite(st).all())
+    for h in range(H):                            # as far apart as the two orders of sums (see above)
+        assert float((out[:, h] - want[:, h]).norm() / want[:, h].norm()) < 3e-6, h
+        assert float((st[:, h] - want_st[:, h]).norm() / want_st[:, h].norm()) < 3e-6, h

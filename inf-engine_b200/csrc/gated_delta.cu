@@ -19,6 +19,7 @@
 // of every sum is fixed by the token and the channel alone, so this kernel's result does not depend on how the
 // sequence was cut into steps or on what else the step holds.  A decode step is a tile of one token.  (The chunked form
 // below sums in another order; the 32-bit path never takes it.)
+#include <cfloat>
 #include "common.cuh"
 
 #if !defined(IE_GD_DK) || !defined(IE_GD_DV)
@@ -603,7 +604,19 @@ __global__ void __launch_bounds__(GD_CT) gated_delta_finish_kernel(GatedDeltaChu
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
   gd_product<4, TN>(acc, qs + r * GD_PK, GD_PK, s0 + cc * GD_PK, GD_PK, 0, GD_DK);
-  gd_product<4, TN>(acc, qk + r * GD_PC, GD_PC, u + cc * GD_PC, GD_PC, 0, GD_C);
+  // a token after t has weight zero for t, which hides it only while its u is a number: with an infinity or NaN in the chunk
+  // the sum ends at t itself, so that a bad token spoils no earlier one
+  bool bad = false;
+  for (int i = tid; i < GD_DV * GD_C; i += GD_CT) bad |= !(fabsf(u[(i / GD_C) * GD_PC + i % GD_C]) <= FLT_MAX);
+  if (__syncthreads_or(bad) == 0) {
+    gd_product<4, TN>(acc, qk + r * GD_PC, GD_PC, u + cc * GD_PC, GD_PC, 0, GD_C);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+        for (int x = 0; x <= r + 16 * i; ++x) acc[i][j] = fmaf(qk[(r + 16 * i) * GD_PC + x], u[(cc + 16 * j) * GD_PC + x], acc[i][j]);
+  }
   __syncthreads();
   float* const so = gd_smem;                      // [GD_C][GD_DV + 1], where the operands were (both products have read them)
   static_assert(GD_C * (GD_DV + 1) <= (GD_C + GD_DV) * (GD_PK + GD_PC), "the outputs take the place of the operands");

@@ -106,3 +106,16 @@ def test_a_decay_of_zero():
     for h in range(H):                            # as far apart as the two orders of sums (see above)
         assert float((out[:, h] - want[:, h]).norm() / want[:, h].norm()) < 3e-6, h
         assert float((st[:, h] - want_st[:, h]).norm() / want_st[:, h].norm()) < 3e-6, h
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_a_token_that_is_no_number_spoils_no_earlier_one(value):
+    H, G, dk, dv, N, at = 2, 1, 64, 64, 130, 100
+    clean = inputs(H, G, dk, dv, N, 6)
+    want = both_forms(clean, H, G, dk, dv)[1][0]
+    x = dict(clean, v=clean["v"].clone())
+    x["v"][at, 3] = value                         # one value channel of the first head, in the middle of a chunk
+    out = both_forms(x, H, G, dk, dv)[0][0]
+    assert bool(torch.isnan(out[at, 0, 3])) and bool(torch.isfinite(out[:at]).all()) and bool(torch.isfinite(out[:, 1]).all())
+    assert float((out[:at] - want[:at]).norm() / want[:at].norm()) < 3e-6
+    assert float((out[:, 1] - want[:, 1]).norm() / want[:, 1].norm()) < 3e-6

@@ -30,10 +30,20 @@ from .linear import Linear
 from .registry import register_mixer
 
 
-# When chunks beat a token after another, in us of heads of 64 x 64 (measured): the chain takes 0.6 a token of the longest request, the
-# chunks 40 and 0.25 for each chunk of 64 tokens and head of all requests.  One request of 32 heads from about 85 tokens on
-# (128 tokens: 80 and 56, 2,048: 1,228 and 293); 8 requests of 128 tokens stay a chain (108, in chunks 148).
-CHAIN_US_PER_TOKEN, CHUNKS_US, CHUNKS_US_PER_TOKEN_AND_HEAD = 0.6, 40.0, 0.25 / 64
+def chunks_pay(q_lens, n_heads: int, head_dim: int, v_head_dim: int) -> bool:
+    """Whether a step whose requests bring ``q_lens`` tokens is faster in chunks than token after token.
+
+    Both costs in us, fitted to measurements on a B200 over heads of 32 x 32 to 128 x 128 and steps of one to 33 requests.  The
+    chain walks the longest request (the others beside it).  A chunk costs the same whether it holds 64 tokens or one, per head and
+    by the size of its state, so every decode token of a mixed step counts as a chunk.  Measured, chain against chunks:
+    32 heads of 64 x 64, one request of 64 tokens 41 and 52, 128: 79 and 55, 2,048: 1,224 and 292; 8 requests of 128: 104 and
+    138; a prompt of 200 beside 32 decode tokens 144 and 278; 128 x 128, three prompts of 300: 268 and 367."""
+    size = head_dim * v_head_dim
+    chain = 1.0 if size > 96 * 96 else 0.85 if head_dim <= 32 else 0.6            # a token
+    chunk = 0.05 + 0.6 * size / (128 * 128)                                       # a chunk and head
+    return 45.0 + chunk * n_heads * sum(-(-n // 64) for n in q_lens) < chain * max(q_lens)
+
+
 CHUNK_MAX_SCRATCH = 1 << 28          # floats (1 GB; 20,000 tokens of 32 heads of 64 x 64): longer steps go token after token
 
 
@@ -115,7 +125,7 @@ class GatedDeltaMixer:
         a_pre = proj[:, c0 + self.vw + s.n_heads:]
         mixed = rt.ws.take("gated_delta_mixed", (n, self.vw), rt.act_dtype)
         scratch = None
-        if not rt.exact and CHUNKS_US + CHUNKS_US_PER_TOKEN_AND_HEAD * s.n_heads * n < CHAIN_US_PER_TOKEN * ctx.max_q_len:
+        if not rt.exact and ctx.max_q_len > 1 and chunks_pay(ctx.host["q_lens"], s.n_heads, s.head_dim, s.v_head_dim):
             floats = kernels.gated_delta_scratch_floats(n, ctx.n_requests, s.n_heads, s.head_dim, s.v_head_dim)
             if 0 < floats <= CHUNK_MAX_SCRATCH:
                 scratch = rt.ws.take("gated_delta_chunks", (floats,), torch.float32)

@@ -44,7 +44,18 @@ def chunks_pay(q_lens, n_heads: int, head_dim: int, v_head_dim: int) -> bool:
     return 45.0 + chunk * n_heads * sum(-(-n // 64) for n in q_lens) < chain * max(q_lens)
 
 
-CHUNK_MAX_SCRATCH = 1 << 28          # floats (1 GB; 20,000 tokens of 32 heads of 64 x 64): longer steps go token after token
+CHUNK_MAX_SCRATCH = 1 << 28          # floats (1 GB; about 26,000 tokens of 32 heads of 64 x 64): longer steps go token after token
+
+
+def chunk_scratch(floats: int, device) -> torch.Tensor | None:
+    """Memory for a step in chunks, given back when the layer has run; None where there is none to be had (no chunked form for these
+    heads, a step beyond the limit, a full device), and the step then goes token after token, which needs none."""
+    if not 0 < floats <= CHUNK_MAX_SCRATCH:
+        return None
+    try:
+        return torch.empty(floats, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def conv_state_requirement(taps: int, channels: int, dtype: torch.dtype) -> CacheRequirement:
@@ -126,9 +137,8 @@ class GatedDeltaMixer:
         mixed = rt.ws.take("gated_delta_mixed", (n, self.vw), rt.act_dtype)
         scratch = None
         if not rt.exact and ctx.max_q_len > 1 and chunks_pay(ctx.host["q_lens"], s.n_heads, s.head_dim, s.v_head_dim):
-            floats = kernels.gated_delta_scratch_floats(n, ctx.n_requests, s.n_heads, s.head_dim, s.v_head_dim)
-            if 0 < floats <= CHUNK_MAX_SCRATCH:
-                scratch = rt.ws.take("gated_delta_chunks", (floats,), torch.float32)
+            scratch = chunk_scratch(kernels.gated_delta_scratch_floats(n, ctx.n_requests, s.n_heads, s.head_dim, s.v_head_dim),
+                                    rt.device)
         kernels.gated_delta(conv[:, :self.qk], conv[:, self.qk:2 * self.qk], conv[:, 2 * self.qk:], b_pre, a_pre, gate,
                             self.a_log, self.dt_bias, self.out_gain, state.state, mixed, ctx.q_start, ctx.slots,
                             ctx.n_requests, s.n_heads, s.n_kv_heads, s.head_dim, s.v_head_dim, s.key_eps, s.norm_eps,

@@ -1,6 +1,9 @@
-"""When a step of the gated delta rule goes in chunks: the choice follows what both forms were measured to take."""
+"""When a step of the gated delta rule goes in chunks: the choice follows what both forms were measured to take, and
+a step that finds no memory for chunks goes token after token."""
 import pytest
+import torch
 
+from inf_engine_b200.parts import gated_delta
 from inf_engine_b200.parts.gated_delta import chunks_pay
 
 
@@ -25,3 +28,15 @@ def test_the_faster_form_is_taken(q_lens, heads, dk, dv, chain, chunks):
 def test_decode_tokens_count_as_chunks():
     assert chunks_pay([200], 32, 64, 64) and not chunks_pay([200] + [1] * 32, 32, 64, 64)
     assert not chunks_pay([1] * 64, 32, 64, 64)
+
+
+def test_no_memory_for_chunks_is_no_error(monkeypatch):
+    got = gated_delta.chunk_scratch(1000, "cpu")
+    assert got.numel() == 1000 and got.dtype is torch.float32
+    assert gated_delta.chunk_scratch(0, "cpu") is None and gated_delta.chunk_scratch(gated_delta.CHUNK_MAX_SCRATCH + 1, "cpu") is None
+
+    def full(*args, **kw):
+        raise torch.OutOfMemoryError("CUDA out of memory")
+
+    monkeypatch.setattr(torch, "empty", full)
+    assert gated_delta.chunk_scratch(1000, "cpu") is None

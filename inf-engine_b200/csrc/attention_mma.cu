@@ -21,6 +21,7 @@
 // and the bfloat16 of what that left out, and both parts go through the tensor cores (a weight then carries 16
 // bits of mantissa into a float32 sum), for layers whose weights are to be as exact as their scores.
 #include "common.cuh"
+#include "decode_split.h"
 
 #ifndef IE_ATTN_BIAS
 #define IE_ATTN_BIAS 0
@@ -68,6 +69,7 @@ struct MmaAttnParams {
   int n_heads, n_kv_heads, page_size, window;
   int page_shift;  // log2(page_size) when it is a power of two, else -1
   int split_keys;  // decode: the split of the step's longest request
+  int spread;      // decode: the whole launch has places at once
   float scale_log2;
   // decode with the position encoding and the cache write folded in (every request brings one token):
   // fuse bit 0: q arrives unrotated and is rotated as it is loaded; bit 1: the token's key and value arrive
@@ -666,20 +668,12 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   const int min_first = p.window > 0 ? max(0, ctx - p.window + 1) : 0;
   const int lo_all = (min_first / DC_KT) * DC_KT;
 
-  // This request's own split: its visible keys over all the warps that the launch gives a (request, kv head), in whole tiles,
-  // at least 64 (or the launch's split, if that is shorter).  The launch is cut for the longest request of the step; with its
-  // split for all, a request of a quarter of those keys would leave three warps in four idle (64 requests of 250 to 1,750
-  // keys, heads of 64: 48.8 us a layer with one split for all, 44.0 with each its own).
   const int span = max_lim + 1 - lo_all;
-  const int even = (span + (int)gridDim.x * DC_WARPS - 1) / ((int)gridDim.x * DC_WARPS);
-  const int split_keys = max(min(64, p.split_keys), (even + DC_KT - 1) / DC_KT * DC_KT);
-  const int s_last = (span - 1) / split_keys;
-  const int k_lo = lo_all + split * split_keys;
-  const int k_hi = min(k_lo + split_keys, max_lim + 1);
-  const bool has_work = split <= s_last && n_pairs > 0;
-  // blocks that hold at least one split
-  const int b_first = 0, b_last = s_last / DC_WARPS;
-  const int n_active_blocks = b_last - b_first + 1;
+  const DecodeSplit own = decode_split(span, p.split_keys, (int)gridDim.x, p.spread != 0, DC_WARPS, DC_KT);
+  const int k_lo = lo_all + split * own.keys;
+  const int k_hi = min(k_lo + own.keys, max_lim + 1);
+  const bool has_work = k_lo <= max_lim && n_pairs > 0;
+  const int n_active_blocks = own.blocks;                     // blocks that hold at least one split: the first ones
   // A block without keys leaves at once and frees its slot.  It need not wait for the kernel ahead:
   // block 0 of every (request, kv head) always has keys and waits, so this kernel still ends after it.
   // (a request with more than 16 rows is not this kernel's: in a mixed step the prefill kernel takes it)
@@ -687,7 +681,7 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   // whether the blocks add up inside their cluster: the same answer in every block of the cluster, and every one
   // of them, with keys or without, then meets both cluster barriers below
   const bool merge_in_cluster = p.cluster_merge != 0 && n_active_blocks > 1;
-  if ((int)blockIdx.x < b_first || (int)blockIdx.x > b_last) {
+  if ((int)blockIdx.x >= n_active_blocks) {
     if (merge_in_cluster) {
       cluster_barrier();
       cluster_barrier();
@@ -795,7 +789,7 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   __syncthreads();
   TRACE(6);                                                  // all warps of the block done
   const int n_out = n_pairs * HD;
-  const int blk = (int)blockIdx.x - b_first;
+  const int blk = (int)blockIdx.x;
   for (int idx = threadIdx.x; idx < n_out; idx += DC_THREADS) {
     const int pr = idx / HD, d = idx - pr * HD;
     float M = -INFINITY;
@@ -828,10 +822,10 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   if (n_active_blocks == 1) return;
 
   if (merge_in_cluster) {
-    // ---- the cluster of this (request, kv head): its first block with keys adds the blocks up, in ascending
+    // ---- the cluster of this (request, kv head): its first block adds the blocks up, in ascending
     // order and with the arithmetic of the ticket path below, from the others' shared memory
     cluster_barrier();
-    if ((int)blockIdx.x == b_first) {
+    if (blockIdx.x == 0) {
       const uint32_t res = smem_u32(smem + DC_WARPS * DC_WARP_BYTES);
       for (int idx = threadIdx.x; idx < n_out; idx += DC_THREADS) {
         const int pr = idx / HD, d = idx - pr * HD;
@@ -840,7 +834,7 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
         float v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const uint32_t peer = cluster_map(res, (uint32_t)(b_first + min(u, n_active_blocks - 1)));   // rank == blockIdx.x
+          const uint32_t peer = cluster_map(res, (uint32_t)min(u, n_active_blocks - 1));   // rank == blockIdx.x
           mlv[u] = ld_cluster_f32x2(peer + (16 * HD + pr * 2) * 4);
           v[u] = ld_cluster_f32(peer + (pr * HD + d) * 4);
         }
@@ -938,7 +932,7 @@ static void fill(MmaAttnParams& p, const void* q, void* out, const void* kpool, 
   p.cluster_merge = 0;
   p.q_stride = q_stride; p.out_stride = out_stride; p.table_stride = table_stride;
   p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.page_size = page_size; p.window = window;
-  p.split_keys = 0; p.n_blocks = 0; p.scale_log2 = scale * LOG2E;
+  p.split_keys = 0; p.spread = 0; p.n_blocks = 0; p.scale_log2 = scale * LOG2E;
   p.fuse = 0; p.k_new = nullptr; p.v_new = nullptr; p.kv_stride = 0; p.cos_t = nullptr; p.sin_t = nullptr;
   p.positions = nullptr; p.slot_mapping = nullptr;
   p.score_bias = nullptr; p.bias_dists = 0; p.head_scale = nullptr;
@@ -1080,16 +1074,17 @@ static int decode_launch(MmaAttnParams& p, float* scratch, int n_requests, int n
 #else
   constexpr bool no_cluster = false;
 #endif
-  static int block_places = -1;
+  static int block_places = -1, sms = 0;
   if (block_places < 0) {
     block_places = 0;
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, per_sm = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attention_decode_kernel, DC_THREADS, smem) == cudaSuccess)
       block_places = sms * per_sm;
   }
   const long long launch_blocks = (long long)p.n_blocks * n_kv_heads * n_requests;
+  p.spread = launch_blocks <= 2LL * sms ? 1 : 0;
   p.cluster_merge = (!no_cluster && p.n_blocks >= 2 && p.n_blocks <= 8 && launch_blocks <= block_places) ? 1 : 0;
   dim3 grid(p.n_blocks, n_kv_heads, n_requests);
   return launch_k_cluster(attention_decode_kernel, p.cluster_merge ? p.n_blocks : 1, grid, DC_THREADS, smem, stream, p);

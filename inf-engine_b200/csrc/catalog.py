@@ -13,8 +13,8 @@ def all_build_requests():
     reqs.append(("attn_tcgen05", ["attention_tcgen05.cu"], {}, []))
     reqs.append(("attn_tcgen05_exact", ["attention_tcgen05.cu"], {"IE_FA_EXACT": 1}, []))
     for hd in (64, 128):
-        reqs.append((f"attn_mma_hd{hd}", ["attention_mma.cu"], {"IE_HD": hd}, ["attention_noalloc.h"]))
-        reqs.append((f"attn_mma_hd{hd}_bias", ["attention_mma.cu"], {"IE_HD": hd, "IE_ATTN_BIAS": 1}, ["attention_noalloc.h"]))
+        reqs.append((f"attn_mma_hd{hd}", ["attention_mma.cu"], {"IE_HD": hd}, ["attention_noalloc.h", "decode_split.h"]))
+        reqs.append((f"attn_mma_hd{hd}_bias", ["attention_mma.cu"], {"IE_HD": hd, "IE_ATTN_BIAS": 1}, ["attention_noalloc.h", "decode_split.h"]))
     for dk, dv in ((64, 64), (64, 128), (128, 128)):   # (key, value) head sizes of the float32-score attention worth having early
         reqs.append((f"attn_wide_k{dk}_v{dv}", ["attention_wide.cu"], {"IE_AW_DK": dk, "IE_AW_DV": dv}, []))
     for dk, dv in ((64, 64), (128, 128)):              # the same with capped scores

@@ -1083,7 +1083,7 @@ def attention_mma_library(head_dim: int, biased: bool = False):
         if biased:
             defines["IE_ATTN_BIAS"] = 1
             name += "_bias"
-        lib = load_library(name, ["attention_mma.cu"], defines, ["attention_noalloc.h"])
+        lib = load_library(name, ["attention_mma.cu"], defines, ["attention_noalloc.h", "decode_split.h"])
         P, I, F = c_void_p, c_int, c_float
         lib.ie_attention_prefill_biased.argtypes = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, P, P]
         lib.ie_attention_prefill_biased.restype = c_int

@@ -364,7 +364,7 @@ causal_conv_kernel(const TA* __restrict__ x, int x_stride, const TW* __restrict_
 
 // bfloat16 rows on 16 bytes, filters of up to four taps: a thread takes 8 channels and 8 tokens in a row and keeps the inputs of the
 // filter's length in registers, so a row is read once, 16 bytes a lane (the kernel above reads two bytes a lane and every row
-// `taps` times).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 79 us, 23 so.
+// `taps` times).  The caller says where this pays (`in_runs`: short requests leave most of a run empty).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 79 us, 23 so.
 #define CV_CH 8
 #define CV_RUN 8
 template <typename TW, int TAPS>
@@ -375,6 +375,12 @@ causal_conv_vec_kernel(const bf16* __restrict__ x, int x_stride, const TW* __res
   pdl_trigger();
   const int c = (blockIdx.x * 32 + threadIdx.x) * CV_CH;
   const int req = blockIdx.y;
+  // (cuts and slots are the step's, copied in before its first kernel)
+  const int q0 = q_start[req], q1 = q_start[req + 1];
+  if (q0 + (int)blockIdx.z * CONV_CHUNK >= q1 && blockIdx.z > 0) {           // a shorter request than the step's longest
+    pdl_wait();
+    return;
+  }
   // the filter does not depend on the kernel ahead: asked for before the wait, 16 bytes at a time (a thread's 8 filters lie
   // side by side)
   float wv[TAPS][CV_CH], b[CV_CH];
@@ -392,9 +398,7 @@ causal_conv_vec_kernel(const bf16* __restrict__ x, int x_stride, const TW* __res
       for (int e = 0; e < CV_CH; ++e) b[e] = 0.f;
   }
   pdl_wait();
-  const int q0 = q_start[req], q1 = q_start[req + 1];
   const int t_lo = q0 + blockIdx.z * CONV_CHUNK + threadIdx.y * CV_RUN, t_hi = min(q1, t_lo + CV_RUN);
-  if (q0 + (int)blockIdx.z * CONV_CHUNK >= q1 && blockIdx.z > 0) return;     // a shorter request than the step's longest
   const int slot = IE_SLOT(slots[req]);
   const bool live = c < channels;
   bf16* st = (slot >= 0 && live) ? state + (size_t)slot * state_slot_stride + c : nullptr;   // element i at st[i * channels]
@@ -458,14 +462,13 @@ causal_conv_vec_kernel(const bf16* __restrict__ x, int x_stride, const TW* __res
 extern "C" int ie_causal_conv(const void* x, int x_stride, const void* w, const void* bias, int w_dtype, void* state,
                               long long state_slot_stride, void* out, int out_stride, const int* q_start,
                               const int* slots, int n_requests, int channels, int taps, int activation,
-                              int write_state, int act_dtype, int max_q_len, cudaStream_t stream) {
+                              int write_state, int act_dtype, int max_q_len, int in_runs, cudaStream_t stream) {
   if (n_requests <= 0 || channels <= 0) return IE_OK;
   if (taps < 1 || taps > CONV_MAX_TAPS || max_q_len < 1) return IE_BAD_SIZE;
   const int chunks = (max_q_len + CONV_CHUNK - 1) / CONV_CHUNK;       // of the step's longest request
   if (chunks > 65535) return IE_BAD_SIZE;
   dim3 grid((channels + CONV_CH - 1) / CONV_CH, n_requests, chunks), block(CONV_CH, CONV_TL);
-  // from a run of tokens on: a step of single tokens leaves seven threads in eight of it idle (8 requests: 10.9 us, the kernel above 6.6)
-  const bool vec = act_dtype == IE_BF16 && max_q_len >= CV_RUN && taps >= 2 && taps <= 4 && channels % CV_CH == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 &&
+  const bool vec = in_runs && act_dtype == IE_BF16 && taps >= 2 && taps <= 4 && channels % CV_CH == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 &&
                    state_slot_stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)state | (uintptr_t)w | (uintptr_t)bias) & 15) == 0;
 #define CV_GO(TW, TAPS)                                                                                            \
   return launch_k(causal_conv_vec_kernel<TW, TAPS>, dim3((channels + 32 * CV_CH - 1) / (32 * CV_CH), n_requests, chunks),   \

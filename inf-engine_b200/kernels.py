@@ -104,7 +104,7 @@ def core():
         lib.ie_moe_combine_outnorm.restype = c_int
         lib.ie_outnorm_accumulate_norm.argtypes = [P, P, I, I, P, I, F, P, I, F, P, I, I, I, P]
         lib.ie_outnorm_accumulate_norm.restype = c_int
-        lib.ie_causal_conv.argtypes = [P, I, P, P, I, P, L, P, I, P, P, I, I, I, I, I, I, I, P]
+        lib.ie_causal_conv.argtypes = [P, I, P, P, I, P, L, P, I, P, P, I, I, I, I, I, I, I, I, P]
         lib.ie_attention_rows.argtypes = [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, I, P, I, P, I, I, F, I, I, I, P, F, P, I, P]
         lib.ie_linear_recurrence.argtypes = [P, I, P, I, P, P, I, P, P, P, I, P, P, I, P, P, I, I, F, F, I, I, I, P]
         lib.ie_rownorm_rotate_write.argtypes = [P, P, P, I, I, I, P, P, P, P, P, I, F, P, I, P, P, P, P, I, I, I, I, I, I, I, P]
@@ -516,15 +516,32 @@ def outnorm_accumulate_norm(residual: torch.Tensor, y: torch.Tensor, gain: torch
 CONV_MAX_TAPS = 16
 
 
+def conv_runs_pay(n_tokens: int, n_requests: int, max_q_len: int, channels: int, taps: int) -> bool:
+    """Whether ``causal_conv`` is faster with threads on runs of eight tokens than with a thread a token (bfloat16 rows on 16
+    bytes; measured on a B200 over 64 to 6,144 channels and steps of one to 64 requests).  A run of one token leaves seven
+    eighths of its thread's work unused, so steps of mostly decode tokens stay (a prompt of 100 beside 60 of them, 2,048
+    channels: 30 us, 41 in runs), and a launch in runs is no shorter than 8 us (one request of 16 tokens: 4.5).  With three or four
+    taps runs win from 48 tokens a request (61 of 3,072 channels: 10.1 and 7.8) or enough rows together (8 requests of 24 tokens,
+    2,048 channels: 10.5 and 7.7; 1,024 channels: 6.0 and 7.8); with two, where a token costs less, only from large steps on."""
+    if n_tokens < 10 * n_requests or max_q_len < 16:
+        return False
+    return (max_q_len >= 48 or n_tokens * channels >= 1 << 18) if taps > 2 else n_tokens * channels >= 700_000
+
+
 def causal_conv(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor,
                 q_start: torch.Tensor, slots: torch.Tensor, n_requests: int, activation: str | None = None,
-                write_state: bool = True, max_q_len: int | None = None) -> None:
+                write_state: bool = True, max_q_len: int | None = None, in_runs: bool | None = None) -> None:
     """A causal convolution per channel over each request's tokens of the step: ``out[t, c] = act(bias[c] + sum_j
     weight[c, j] * x[t - (taps - 1 - j), c])``.  ``state`` [slots, taps - 1, channels] (activation type) holds every
     request's last inputs, oldest first, and is moved on by the step's tokens (with ``write_state``).  ``max_q_len``: the
-    most tokens one request brings (the launch is cut for it; the step's token count when not given)."""
+    most tokens one request brings (the launch is cut for it; the step's token count when not given).  ``in_runs``: whether
+    threads take runs of tokens, 16 bytes of a row at a time, where types and alignment allow (the same bits; None:
+    ``conv_runs_pay``)."""
     n, channels = x.shape
     taps = weight.shape[1]
+    max_q_len = int(max_q_len) if max_q_len else max(n, 1)
+    if in_runs is None:
+        in_runs = conv_runs_pay(n, n_requests, max_q_len, channels, taps)
     assert weight.shape == (channels, taps) and weight.is_contiguous() and x.stride(1) == 1 and out.stride(1) == 1
     assert out.shape == (n, channels) and out.dtype == x.dtype and state.dtype == x.dtype and state.stride(-1) == 1
     assert state.shape[1:] == (max(taps - 1, 0), channels) and (taps == 1 or state.stride(1) == channels)
@@ -533,7 +550,7 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
     _check(core().ie_causal_conv(_ptr(x), x.stride(0), _ptr(weight), _ptr(bias), dtype_code(weight.dtype), _ptr(state),
                                  state.stride(0), _ptr(out), out.stride(0), _ptr(q_start), _ptr(slots), n_requests,
                                  channels, taps, {None: 0, "silu": 1}[activation], 1 if write_state else 0,
-                                 dtype_code(x.dtype), int(max_q_len) if max_q_len else max(n, 1), _stream()),
+                                 dtype_code(x.dtype), max_q_len, 1 if in_runs else 0, _stream()),
            f"causal_conv(channels={channels}, taps={taps})")
 
 

@@ -160,7 +160,8 @@ def test_experts_of_a_few_tokens_through_the_ring(epi, tokens, experts, top, hid
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n,d,top,shared,gated", [(1, 8, 1, True, True), (3, 2048, 2, True, True), (2, 2056, 3, False, False), (2, 8192, 2, True, True)])
+@pytest.mark.parametrize("n,d,top,shared,gated", [(1, 8, 1, True, True), (3, 2048, 2, True, True), (2, 2056, 3, False, False), (2, 8192, 2, True, True),
+                                                  (5, 64, 2, True, True), (3, 256, 3, True, True), (2, 264, 1, False, False)])
 def test_mixture_normed_into_the_stream(dtype, n, d, top, shared, gated):
     from inf_engine_b200 import kernels as k
     y, w, res = rnd(1, n * top, d), rnd(2, n, top).abs(), rnd(3, n, d)

@@ -131,7 +131,7 @@ class RoutedExperts:
             kernels.gemm_tcgen05_grouped(hidden, self.down, y, tiles, sorted_pairs, "f32")
             return y, weights, gate
         if (rt.act_dtype is torch.bfloat16 and self.first.dtype is torch.bfloat16 and self.down.dtype is torch.bfloat16
-                and kernels.moe_ring_supports(x, s.hidden, s.intermediate)):
+                and kernels.moe_ring_pays(s.hidden, s.intermediate) and kernels.moe_ring_supports(x, s.hidden, s.intermediate)):
             rows = kernels.MOE_RING_ROWS
             tiles = ws.take("moe_tiles", (kernels.moe_max_tiles(n_pairs, E, rows), 4), torch.int32)
             kernels.moe_sort(ids, E, sorted_pairs, tiles, rows)

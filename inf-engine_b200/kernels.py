@@ -431,7 +431,11 @@ def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
            f"gemm_simt_batched({a.dtype},{w.dtype}, blocks={blocks})")
 
 
-DIAG_FEW_ROWS = 16      # up to here a warp an output column beats tiles of 64 rows
+def diag_rows_pay(m: int, k: int) -> bool:
+    """Whether a warp an output column beats tiles of 64 rows in a block-diagonal product: up to 16 rows, and k long enough for
+    the warp's trees at the end (8 rows of blocks of 256: 15.3 us in tiles, 5.1 so; of 64: 4.7 and 3.4, 16 rows 4.9 and 5.7; of 16:
+    2.1 and 3.4)."""
+    return m <= 16 and k >= 64 and 8 * m <= k
 
 
 def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
@@ -445,7 +449,7 @@ def block_diagonal(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     assert a.shape[1] == blocks * k and out.shape == (m, blocks * n) and out.dtype is torch.float32
     assert a.stride(1) == 1 and w.is_contiguous() and out.stride(1) == 1
     aligned = a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-    few = a.dtype is torch.bfloat16 and m <= DIAG_FEW_ROWS
+    few = a.dtype is torch.bfloat16 and diag_rows_pay(m, k)
     if few and k % 4 == 0 and a.stride(0) % 4 == 0 and aligned:
         _check(core().ie_gemm_diag_rows(_ptr(a), dtype_code(a.dtype), _ptr(w), dtype_code(w.dtype), _ptr(out), m, blocks, n, k,
                                         a.stride(0), out.stride(0), _stream()), f"gemm_diag_rows(blocks={blocks}, n={n}, k={k})")

@@ -8,3 +8,10 @@ from inf_engine_b200 import kernels
 @pytest.mark.parametrize("hidden,inter,blocks,ring", [(256, 256, 10.5, 11.6), (512, 256, 13.0, 13.5), (1024, 512, 58.0, 36.2), (1024, 1024, 37.4, 25.0), (2048, 2048, 82.2, 60.1)])
 def test_experts_through_the_ring(hidden, inter, blocks, ring):
     assert kernels.moe_ring_pays(hidden, inter) == (ring < blocks)
+
+
+# a block-diagonal product, us: (rows, k of a block, tiles of 64 rows, a warp an output)
+@pytest.mark.parametrize("m,k,tiles,warps", [(8, 256, 15.3, 5.1), (16, 256, 15.4, 8.7), (1, 64, 4.7, 2.6), (8, 64, 4.7, 3.4), (16, 64, 4.9, 5.7),
+                                             (4, 16, 2.1, 2.8), (16, 16, 2.2, 5.4), (16, 512, 36.7, 24.8), (17, 256, 15.7, 16.0)])
+def test_gate_products_of_a_few_rows(m, k, tiles, warps):
+    assert kernels.diag_rows_pay(m, k) == (warps < tiles)

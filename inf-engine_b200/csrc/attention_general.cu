@@ -711,9 +711,11 @@ extern "C" int ie_attention_ordered_rows(const void* q, void* out, const void* k
   const dim3 grid(n_tokens, n_heads);
 #define AO_GO(T, VEC)                                                                                                      \
   {                                                                                                                        \
-    static const cudaError_t e = cudaFuncSetAttribute(attention_ordered_rows_kernel<T, VEC>,                               \
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);             \
-    if (e != cudaSuccess) return (int)e;                                                                                   \
+    static OncePerDevice once;                                                                                             \
+    const int ready = once([] {                                                                                            \
+      return cudaFuncSetAttribute(attention_ordered_rows_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); \
+    });                                                                                                                    \
+    if (ready) return ready;                                                                                               \
     return launch_k(attention_ordered_rows_kernel<T, VEC>, grid, AO_THREADS, smem, stream, p, n_requests, max_rows, tiles); \
   }
   if (act_dtype == IE_F32 && vec) AO_GO(float, true);

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include <atomic>
 #include <tuple>
 #include <utility>
 
@@ -124,6 +125,34 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 #define TANH_COEFS 0.99999994f, -0.333327681f, 0.133204684f, -0.0527566522f, 0.0167278275f
 
 static inline int launch_status() { return (int)cudaGetLastError(); }
+
+// What has to be done once on every device, such as raising a kernel's limit of dynamic shared memory: a program may run
+// models on several GPUs, and a setting of one says nothing about the next.  A failure is not remembered.
+struct OncePerDevice {
+  std::atomic<unsigned long long> done{0};      // a bit a device (beyond 64 devices: done at every call)
+  template <typename F>
+  int operator()(F set) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (done.load(std::memory_order_relaxed) & bit) return 0;
+    const int rc = (int)set();
+    if (rc == 0) done.fetch_or(bit, std::memory_order_relaxed);
+    return rc;
+  }
+};
+
+// SMs of the current device (0: it did not say)
+static inline int device_sms() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
 
 // ---------------------------------------------------- programmatic dependent launch
 // Every kernel of this package is launched so that it may start while the kernel

@@ -646,15 +646,16 @@ constexpr size_t GD_FINISH_SMEM = (size_t)(GD_C * GD_PK + GD_DV * GD_PK + GD_C *
 
 template <typename TA, typename TW>
 static int gd_launch_chunks(const GatedDeltaChunks& d, int n_requests, int chunks, cudaStream_t stream) {
-  static const cudaError_t ready = [] {
+  static OncePerDevice once;
+  const int ready = once([] {
     cudaError_t e = cudaFuncSetAttribute(gated_delta_prepare_kernel<TA, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_PREPARE_SMEM);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(gated_delta_carry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_CARRY_SMEM);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(gated_delta_finish_kernel<TA, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_FINISH_SMEM);
     return e;
-  }();
-  if (ready != cudaSuccess) return (int)ready;
+  });
+  if (ready) return ready;
   const dim3 grid(chunks, d.p.n_heads, n_requests);
   int rc = launch_k(gated_delta_prepare_kernel<TA, TW>, grid, GD_CT, GD_PREPARE_SMEM, stream, d);
   if (!rc) rc = launch_k(gated_delta_carry_kernel, dim3(GD_DV / GD_SLICE, d.p.n_heads, n_requests), GD_CARRY_T, GD_CARRY_SMEM, stream, d);

@@ -327,7 +327,8 @@ int gf_allow_smem(K kernel, size_t smem) {
 template <int NR, int MR, int STAGES, int CL>
 int launch_stream(const GfParams& p, int max_clusters, cudaStream_t stream) {
   constexpr size_t smem = (size_t)(GF_PARTS / CL) * STAGES * (16 * NR + 2 * MR) * GF_PITCH * 4;
-  static const int ready = gf_allow_smem(gemm_f32_stream_kernel<NR, MR, STAGES, CL>, smem);
+  static OncePerDevice once;
+  const int ready = once([] { return gf_allow_smem(gemm_f32_stream_kernel<NR, MR, STAGES, CL>, smem); });
   if (ready) return ready;
   const int groups = (p.N + 16 * NR - 1) / (16 * NR);
   const int grid = (max_clusters > 0 && groups > max_clusters ? max_clusters : groups) * CL;
@@ -339,7 +340,8 @@ int launch_stream(const GfParams& p, int max_clusters, cudaStream_t stream) {
 template <int TM, bool SPLIT>
 int launch_tile(const GfParams& p, int tiles, cudaStream_t stream) {
   constexpr size_t smem = ((size_t)GF_TILE_STAGES * (8 * TM + GF_BN) * GF_PITCH + 8 * TM * GF_BN) * 4;
-  static const int ready = gf_allow_smem(gemm_f32_tile_kernel<TM, SPLIT>, smem);
+  static OncePerDevice once;
+  const int ready = once([] { return gf_allow_smem(gemm_f32_tile_kernel<TM, SPLIT>, smem); });
   if (ready) return ready;
   if (SPLIT) return launch_k_cluster(gemm_f32_tile_kernel<TM, SPLIT>, GF_PARTS, tiles * GF_PARTS, GF_TILE_THREADS, smem, stream, p);
   return launch_k(gemm_f32_tile_kernel<TM, SPLIT>, tiles, GF_TILE_THREADS, smem, stream, p);
@@ -355,12 +357,8 @@ int gemm_f32_takes(const void* A, const void* W, int K, int lda, int ldw) {
 }
 
 int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-  static int n_sms = 0;
-  if (!n_sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      return IE_BAD_SIZE;
-  }
+  const int n_sms = device_sms();
+  if (n_sms <= 0) return IE_BAD_SIZE;
   GfParams p;
   p.A = A; p.W = W; p.C = C; p.M = M; p.N = N; p.K = K; p.lda = lda; p.ldw = ldw; p.ldc = ldc;
   p.part = (((K + GF_PARTS - 1) / GF_PARTS) + GF_BK - 1) / GF_BK * GF_BK;

@@ -769,9 +769,9 @@ __global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
 
 template <int NT, int EPI>
 int launch_ring(const GroupedParams& p, int n_sms, size_t smem, cudaStream_t stream) {
-  static const cudaError_t ready =
-      cudaFuncSetAttribute(moe_ring_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024);
-  if (ready != cudaSuccess) return (int)ready;
+  static OncePerDevice once;
+  const int ready = once([] { return cudaFuncSetAttribute(moe_ring_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024); });
+  if (ready) return ready;
   return launch_k(moe_ring_kernel<NT, EPI>, n_sms, THREADS, smem, stream, p);
 }
 

@@ -681,10 +681,7 @@ extern "C" int ie_linear_recurrence(const void* u, int u_stride, const void* y_p
                                     cudaStream_t stream) {
   if (n_requests <= 0 || width <= 0) return IE_OK;
   dim3 grid((width + 127) / 128, n_requests), run_grid((width + LS_CH - 1) / LS_CH, n_requests);
-  static const int n_sms = [] {
-    int dev = 0, v = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? v : 1;
-  }();
+  const int n_sms = max(1, device_sms());
   const long long rounds = ((long long)run_grid.x * n_requests + n_sms - 1) / n_sms;
 #define LRU_GO(TA, TW)                                                                                             \
   if (max_q_len >= LS_MIN_TOKENS * rounds)                                                                         \

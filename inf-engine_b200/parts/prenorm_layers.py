@@ -5,7 +5,7 @@ with the same operands.  Issued from Python such a step is bound by the host up 
 Which models: every block pre-norm with RMS norms, attention without options beside a rotation table and a window, a silu
 feed-forward, bfloat16 throughout, all layers of one geometry, nothing done to the stream between them.  Which steps: more
 rows than the streaming products take, and at least one request that brings more than one token (steps of decode tokens
-alone are graphs).  Sizes and pointers are read anew for every step; nothing is kept from one to the next."""
+alone are graphs), with ``torch.mm`` left at its own defaults.  Sizes and pointers are read anew for every step; nothing is kept from one to the next."""
 
 from __future__ import annotations
 
@@ -51,6 +51,13 @@ def _library_product() -> int:
     return _gemm_ex
 
 
+def _torch_product_is_plain() -> bool:
+    """Whether ``torch.mm`` would call that very product with the handle's standing settings.  A program can ask for full-precision
+    partial sums, another library or tuned kernels, and ``torch.mm`` looks at all three on every call."""
+    return (torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction is True and not torch.cuda.tunable.is_enabled()
+            and torch.backends.cuda.preferred_blas_library() == torch._C._BlasBackend.Cublas)
+
+
 def _address(fn) -> int:
     return ctypes.cast(fn, c_void_p).value
 
@@ -94,7 +101,8 @@ class NativeLayers:
         return cls(blocks, list(views[:len(blocks)]), rt)
 
     def takes(self, ctx) -> bool:
-        return ctx.n_tokens > kernels.STREAM_BEST_ROWS and ctx.max_q_len > 1 and "graph" not in ctx.host and _library_product() != 0
+        return ctx.n_tokens > kernels.STREAM_BEST_ROWS and ctx.max_q_len > 1 and "graph" not in ctx.host and _torch_product_is_plain() \
+            and _library_product() != 0
 
     def forward(self, residual: torch.Tensor, pending, ctx):
         """``(residual, delta)`` after the last layer, as its block would return them."""

@@ -10,6 +10,7 @@ alone are graphs), with ``torch.mm`` left at its own defaults.  Sizes and pointe
 from __future__ import annotations
 
 import ctypes
+import os
 from ctypes import c_float, c_int, c_void_p
 
 import torch
@@ -41,11 +42,17 @@ _gemm_ex: int | None = None
 
 
 def _library_product() -> int:
-    """The address of the matrix product that ``torch.mm`` calls for bfloat16 operands (0: not found)."""
+    """The address of the matrix product that ``torch.mm`` calls for bfloat16 operands (0: not found).  It gets PyTorch's own
+    handle, so it has to come from the library that PyTorch has loaded: a library of the same name that only lies on the path
+    is not opened, nor one of another major version than PyTorch was built for."""
     global _gemm_ex
     if _gemm_ex is None:
         try:
-            _gemm_ex = ctypes.cast(ctypes.CDLL("libcublas.so.12").cublasGemmEx, c_void_p).value or 0
+            major = (torch.version.cuda or "").split(".")[0]
+            if major != "12":              # the types of the call (parts of the library's interface) are those of version 12
+                raise OSError("PyTorch is built for another version of the library")
+            lib = ctypes.CDLL("libcublas.so.12", mode=os.RTLD_NOLOAD | os.RTLD_NOW)
+            _gemm_ex = ctypes.cast(lib.cublasGemmEx, c_void_p).value or 0
         except (OSError, AttributeError):
             _gemm_ex = 0
     return _gemm_ex

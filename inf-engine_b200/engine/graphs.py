@@ -6,14 +6,15 @@ dominate at small batch.  The reference does the same with
 ``torch.cuda.CUDAGraph`` per (batch, length) bucket and ``.copy_()`` into static
 tensors (engine/llama_paged_engine.py:288-415).
 
-Here a graph is kept per (batch bucket, block-table width, longest context, with or without sampling).  Everything that
+Here a graph is kept per (batch bucket, block-table width, longest context).  Everything that
 changes from step to step — token ids, positions, lengths, page slots, block
 tables, sampling records — sits in one static int32 buffer that is refilled by
 a single copy from pinned memory before each replay; kernels read lengths and
 tables from it, so one graph serves every context length.  Rows beyond the
 live requests are padding: length 0, no page, their results are ignored.
-A step that asks for token ids has the sampling kernel in its graph; one that asks for logits alone does not read them again
-(9 us for one request, 18 for 64 of a vocabulary of 128,256).
+The sampling kernel is in the graph if the step that it was captured for asked for token ids: a program that asks for logits
+alone does not have them read again (9 us for one request, 18 for 64 of a vocabulary of 128,256).  A graph serves both kinds of step
+all the same: without the kernel in it, a step that asks for token ids launches the kernel behind it.
 """
 
 from __future__ import annotations
@@ -52,6 +53,7 @@ class _Captured:
     def __init__(self):
         self.graph = None
         self.generation = -1
+        self.sampling = False       # whether the graph holds the sampling kernel
 
 
 KEYS_STEP = 256      # graphs are captured per this many keys of the longest context (more when it is long: keys_bucket)
@@ -94,8 +96,8 @@ class DecodeGraphs:
         n += B
         return off, n
 
-    def _get(self, B: int, widths: tuple[int, ...], keys_hint: int, sampling: bool):
-        key = (B, widths, keys_hint, sampling)
+    def _get(self, B: int, widths: tuple[int, ...], keys_hint: int):
+        key = (B, widths, keys_hint)
         b = self._buckets.get(key)
         if b is not None:
             self._buckets[key] = self._buckets.pop(key)       # most recently used last
@@ -103,7 +105,7 @@ class DecodeGraphs:
             while len(self._buckets) >= MAX_GRAPHS:
                 self._buckets.pop(next(iter(self._buckets)))
             b = _Captured()
-            b.B, b.widths, b.sampling = B, widths, sampling
+            b.B, b.widths = B, widths
             b.off, b.n = self._layout(B, widths)
             b.dev = torch.zeros(b.n, dtype=torch.int32, device=self.rt.device)
             b.host = np.zeros(b.n, dtype=np.int32)
@@ -187,7 +189,7 @@ class DecodeGraphs:
         # the split-key attention is cut for the longest context of the step, in steps of KEYS_STEP keys: a
         # graph serves until some request has grown past its step
         keys_hint = keys_bucket(max(cache.lengths[e.rid] for e in entries) + 1)
-        b = self._get(B, widths, keys_hint, sample_rows is not None)
+        b = self._get(B, widths, keys_hint)
         self._fill(b, entries, sample_rows, token_src)
         if device_tokens is not None:
             if token_src is None:
@@ -201,6 +203,7 @@ class DecodeGraphs:
         try:
             ran = False
             if b.graph is None or b.generation != self.generation:
+                b.sampling = sample_rows is not None
                 # One pass outside capture sizes the buffers and builds the work lists; it is also this step's real
                 # run: a model with state per request (a recurrent mixer, the last token of a sequence) must see
                 # every token once, so the graph captured after it is first replayed by the NEXT step it serves.
@@ -248,6 +251,8 @@ class DecodeGraphs:
                 b.graph.replay()                  # capture recorded the launches; this runs them
                 kernels.LAUNCHES += b.n_kernels
                 self.replays += 1
+                if sample_rows is not None and not b.sampling:
+                    kernels.sample(b.logits, b.rows, b.sampled)
         finally:
             rt.ws = saved
         return b.logits[:R], (b.sampled[:R] if sample_rows is not None else None)

@@ -247,11 +247,29 @@ class PagedAttention:
         group = s.n_heads // s.n_kv_heads
         if not (self.rt.act_dtype is torch.bfloat16 and s.head_dim in kernels.MMA_HEAD_DIMS):
             return False
-        if ctx.max_q_len * group < TCGEN05_MIN_ROWS or ctx.max_q_len * group <= 16:
-            return False
-        if not kernels.attention_tcgen05_supports(s.head_dim, ctx.page_size, s.window):
-            return False
-        return ctx.keys_of_small_requests(group, 16)[0] == 0
+        return self.portions_on_tcgen05(ctx) and ctx.max_q_len * group > 16 and ctx.keys_of_small_requests(group, 16)[0] == 0
+
+    # How a step's requests are dealt out to the tensor-core kernels (``_attend``; the native launches ask the same).
+    def portions_on_tcgen05(self, ctx) -> bool:
+        """Whether prompt portions run on tcgen05 tiles (else on mma.sync tiles of ``PORTION_ROWS`` rows)."""
+        s = self.spec
+        return (ctx.max_q_len * (s.n_heads // s.n_kv_heads) >= TCGEN05_MIN_ROWS
+                and kernels.attention_tcgen05_supports(s.head_dim, ctx.page_size, s.window))
+
+    def small_requests(self, ctx, extras: bool) -> tuple[int, int]:
+        """How many requests the split-key kernel takes, those of at most 16 rows, and the most keys one of them holds."""
+        s = self.spec
+        group = s.n_heads // s.n_kv_heads
+        n_small, keys = (ctx.n_requests, ctx.keys_cap) if ctx.max_q_len * group <= 16 else ctx.keys_of_small_requests(group, 16)
+        if ctx.n_requests * s.n_kv_heads > kernels.attention_decode_ticket_words(s.head_dim, extras):
+            n_small = 0        # more (request, kv head) pairs than the split-key kernel has tickets for
+        return n_small, keys
+
+    def split_keys(self, n_small: int, keys: int, extras: bool) -> tuple[int, int]:
+        """The split-key kernel's launch for that many requests: (number of splits, keys per split)."""
+        s = self.spec
+        return decode_splits(keys, n_small * s.n_kv_heads, *kernels.attention_decode_geometry(s.head_dim, extras),
+                             block_slots=2 * kernels.sm_count())
 
     def _decode_scratch(self, ctx, n_splits: int) -> torch.Tensor:
         s = self.spec
@@ -268,16 +286,11 @@ class PagedAttention:
                 and (not extras or group <= 16) and not self.keep_first and self.out_scale == 1.0 and not self.row_mode):
             extra = dict(score_bias_log2e=self._bias_log2e(bias), head_scale=head_scale) if extras else {}
             # tensor-core kernels, built for this head size when first used
-            n_small, small_keys = (ctx.n_requests, ctx.keys_cap) if ctx.max_q_len * group <= 16 \
-                else ctx.keys_of_small_requests(group, 16)
-            if ctx.n_requests * s.n_kv_heads > kernels.attention_decode_ticket_words(s.head_dim, extras):
-                n_small = 0        # more (request, kv head) pairs than the split-key kernel has tickets for
+            n_small, small_keys = self.small_requests(ctx, extras)
             if n_small:
                 # requests with at most 16 rows (decode tokens, as a rule): the split-key kernel; in a mixed step
                 # it leaves the others alone, and the prefill kernel below is given those only
-                n_splits, split_keys = decode_splits(small_keys, n_small * s.n_kv_heads,
-                                                      *kernels.attention_decode_geometry(s.head_dim, extras),
-                                                      block_slots=2 * kernels.sm_count())
+                n_splits, split_keys = self.split_keys(n_small, small_keys, extras)
                 scratch = self._decode_scratch(ctx, n_splits)
                 kernels.attention_decode_mma(q, out, cache.k, cache.v, kvctx.block_table, ctx.q_start,
                                              ctx.ctx_before, scratch, ctx.n_requests, ctx.n_tokens, s.n_heads,
@@ -286,19 +299,17 @@ class PagedAttention:
             if n_small == ctx.n_requests:
                 return
             more_than = 16 if n_small else 0
-            if (not extras and ctx.max_q_len * group >= TCGEN05_MIN_ROWS
-                    and kernels.attention_tcgen05_supports(s.head_dim, ctx.page_size, s.window)):
+            if not extras and self.portions_on_tcgen05(ctx):
                 # prompt portions: tcgen05 tensor cores, tiles of 128 rows by 128 keys
                 work_req, work_pair0, n_work = ctx.attention_work(group, 128, more_than)
                 kernels.attention_tcgen05(q, out, cache.k, cache.v, kvctx.block_table, ctx.q_start, ctx.ctx_before,
                                           work_req, work_pair0, n_work, s.n_heads, s.n_kv_heads, s.head_dim,
                                           ctx.page_size, self.scale, *rotate)
             else:
-                rows = 64      # tiles of 128 rows (8 warps) leave one block per SM at this register count: slower
-                work_req, work_pair0, n_work = ctx.attention_work(group, rows, more_than)
+                work_req, work_pair0, n_work = ctx.attention_work(group, PORTION_ROWS, more_than)
                 kernels.attention_prefill_mma(q, out, cache.k, cache.v, kvctx.block_table, ctx.q_start,
                                               ctx.ctx_before, work_req, work_pair0, n_work, s.n_heads,
-                                              s.n_kv_heads, s.head_dim, ctx.page_size, s.window, self.scale, rows,
+                                              s.n_kv_heads, s.head_dim, ctx.page_size, s.window, self.scale, PORTION_ROWS,
                                               **extra)
             return
         # float32 arithmetic on CUDA cores: requests that bring at most 16 rows (decode tokens) get a block per (token,
@@ -338,6 +349,7 @@ class PagedAttention:
 
 # fewer (token, head-in-group) rows than this in every request: the 64-row mma.sync tiles waste less
 TCGEN05_MIN_ROWS = 128
+PORTION_ROWS = 64      # rows of an mma.sync tile (tiles of 128 rows, 8 warps, leave one block per SM at this register count: slower)
 
 
 def decode_splits(keys: int, n_streams: int, warps_per_block: int = 6, max_blocks: int = 64,

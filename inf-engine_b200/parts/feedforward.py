@@ -68,13 +68,17 @@ class GatedMLP:
 
     TCGEN05_MIN_ROWS = 128     # below one tile of rows the library product is the better choice
 
+    def gate_up_on_tcgen05(self, n: int, x_stride: int) -> bool:
+        s, w = self.spec, self.gate_up.weight
+        return (self.rt.act_dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and n >= self.TCGEN05_MIN_ROWS
+                and kernels.gemm_tcgen05_supports(n, 2 * s.intermediate, s.hidden, x_stride, w.stride(0)))
+
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         n = x.shape[0]
         s, ws, dt = self.spec, self.rt.ws, self.rt.act_dtype
         h = ws.take("ff_hidden", (n, s.intermediate), dt)
         w = self.gate_up.weight
-        if (dt is torch.bfloat16 and w.dtype is torch.bfloat16 and n >= self.TCGEN05_MIN_ROWS
-                and kernels.gemm_tcgen05_supports(n, 2 * s.intermediate, s.hidden, x.stride(0), w.stride(0))):
+        if self.gate_up_on_tcgen05(n, x.stride(0)):
             # gate/up on the tcgen05 tensor cores with the gated activation in the epilogue: the [n, 2*intermediate]
             # matrix never goes to memory
             kernels.gemm_tcgen05(x, w, h, "silu_mul", act=None if self.plain_silu else self.act)

@@ -16,7 +16,7 @@ from ctypes import c_float, c_int, c_void_p
 import torch
 
 from .. import kernels
-from .attention import TCGEN05_MIN_ROWS, PagedAttention, decode_splits
+from .attention import PORTION_ROWS, PagedAttention
 from .block import PreNormBlock
 from .feedforward import GatedMLP
 from .norms import RMSNorm
@@ -127,26 +127,23 @@ class NativeLayers:
         st.qkv, st.attn_out = ptr(qkv), ptr(ws.take("attn_out", (n, a.out_width), bf))
         st.mixer_out, st.ff_out = ptr(ws.take("mixer_out", (n, s.hidden), bf)), ptr(ff_out)
         st.hidden = ptr(ws.take("ff_hidden", (n, inter), bf))
-        if n >= f.TCGEN05_MIN_ROWS and kernels.gemm_tcgen05_supports(n, 2 * inter, s.hidden, s.hidden, s.hidden):
+        if f.gate_up_on_tcgen05(n, s.hidden):
             st.gemm_silu = _address(kernels.tcgen05_library().ie_gemm_tcgen05_act)
         else:
             st.gate_up = ptr(ws.take("ff_gate_up", (n, 2 * inter), bf))
         st.cos_t, st.sin_t, st.positions = ptr(cos), ptr(sin), ptr(ctx.positions)
         st.slot_mapping, st.block_table, st.q_start, st.ctx_before = (ptr(t) for t in (kv.slot_mapping, kv.block_table, ctx.q_start, ctx.ctx_before))
         st.rotate_q = 0 if a._portions_only_on_tcgen05(ctx) else 1
-        # the requests of at most 16 rows on the split-key kernel, the others on tiles (PagedAttention._attend)
-        n_small, keys = (ctx.n_requests, ctx.keys_cap) if ctx.max_q_len * group <= 16 else ctx.keys_of_small_requests(group, 16)
-        if ctx.n_requests * s.n_kv_heads > kernels.attention_decode_ticket_words(s.head_dim, False):
-            n_small = 0
+        # the requests of at most 16 rows on the split-key kernel, the others on tiles, as PagedAttention deals them out
+        n_small, keys = a.small_requests(ctx, False)
         if n_small:
-            st.n_splits, st.split_keys = decode_splits(keys, n_small * s.n_kv_heads, *kernels.attention_decode_geometry(s.head_dim, False),
-                                                       block_slots=2 * kernels.sm_count())
+            st.n_splits, st.split_keys = a.split_keys(n_small, keys, False)
             st.scratch = ptr(a._decode_scratch(ctx, st.n_splits))
             st.attn_small = _address(kernels.attention_mma_library(s.head_dim).ie_attention_decode)
         if n_small < ctx.n_requests:
-            on_tc = ctx.max_q_len * group >= TCGEN05_MIN_ROWS and kernels.attention_tcgen05_supports(s.head_dim, ctx.page_size, s.window)
-            st.mma_rows = 64
-            work_req, work_pair0, st.n_work = ctx.attention_work(group, 128 if on_tc else 64, 16 if n_small else 0)
+            on_tc = a.portions_on_tcgen05(ctx)
+            st.mma_rows = PORTION_ROWS
+            work_req, work_pair0, st.n_work = ctx.attention_work(group, 128 if on_tc else PORTION_ROWS, 16 if n_small else 0)
             st.work_req, st.work_pair0 = ptr(work_req), ptr(work_pair0)
             if on_tc:
                 st.attn_tc = _address(kernels.attention_tcgen05_library().ie_attention_tcgen05)

@@ -710,6 +710,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
   // consumers: a warp takes an eighth of every stage's k
   const int g = lane >> 2, t = lane & 3;
   const int kw = warp * (p.ks / CONSUMER_WARPS), chunks = p.ks / (CONSUMER_WARPS * 32);
+  constexpr int MAX_PIECES = 1024 / (CONSUMER_WARPS * 32);      // a stage holds at most 1,024 k
   int parity = 0, n_done = 0, tile_now = -1;
   const bf16 *xa = p.A, *xb = p.A;
   bool va = false, vb = false, dead = false;
@@ -728,9 +729,9 @@ __global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
     float acc[NT][2][4] = {};
     for (int ksi = 0; ksi < k_stages; ++ksi) {
       // the activations come from L2 and do not depend on the stage: asked for before the wait
-      uint4 x0[8], x1[8];
+      uint4 x0[MAX_PIECES], x1[MAX_PIECES];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < MAX_PIECES; ++c) {
         x0[c] = (va && c < chunks) ? __ldcg(reinterpret_cast<const uint4*>(xa + ksi * p.ks + c * 32)) : make_uint4(0u, 0u, 0u, 0u);
         x1[c] = (vb && c < chunks) ? __ldcg(reinterpret_cast<const uint4*>(xb + ksi * p.ks + c * 32)) : make_uint4(0u, 0u, 0u, 0u);
       }
@@ -741,7 +742,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
       if (!dead) {
         const uint32_t wbase = ring + s * slot_bytes + g * w_pitch + (kw + t * 8) * 2;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < MAX_PIECES; ++c) {
           if (c < chunks) {
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {

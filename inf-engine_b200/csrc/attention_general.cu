@@ -98,8 +98,7 @@ __device__ __forceinline__ void ag_stage16(float* dst, const bf16* src, bool the
 
 // VEC: head sizes that are multiples of 8 with keys and values on 16 bytes.  Staging, scores and the weighted sum then move
 // 16 bytes at a time (element by element they were bound by reads of shared memory, two a product).  Every sum keeps its
-// order, so both forms give the same bits.  300 tokens of 32 heads of 64 in
-// float32: 145 us a layer element by element, 90 so (inside a step, waits for the kernel ahead included).
+// order, so both forms give the same bits.  300 tokens of 32 heads of 64 in float32: 162 us element by element, 86 so.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(AG_THREADS) attention_general_kernel(AttnGeneralParams p) {
   extern __shared__ __align__(16) float smem[];
@@ -556,12 +555,12 @@ extern "C" int ie_attention_rows(const void* q, void* out, const void* kpool, co
 
 // ------------------------------------------------------------------ few rows a request, in the tile kernel's order of sums
 // The tile kernel gives a decode token one block a kv head, of whose 32 rows `group` exist, and walks the keys tile by tile with
-// every latency in the chain: 200 us a layer for 4 requests at 300 keys.  Here a block takes a (token, query head) and 32 to
+// every latency in the chain: 134 us for 4 requests at 300 keys, 32 heads of 64.  Here a block takes a (token, query head) and 32 to
 // 256 keys at a time (as many as their values fit AO_VALUES floats): values on their way to shared memory, a thread a key for
 // the scores, a warp a tile for maxima, weights and their sums, and a thread a dimension for the output.  Every dot
 // product, maximum, weight and sum is formed as the tile kernel forms it (tiles of 32 keys at multiples of 32, ascending),
-// so that a sequence gives the same bits however it was cut into steps.  Same 4 requests: 188 us a layer less (a step of 16
-// layers 4,857 -> 1,852 us).
+// so that a sequence gives the same bits however it was cut into steps.  Same 4 requests: 21 us (one
+// request at 4,000 keys 1,646 and 169).
 #define AO_THREADS 256
 #define AO_VALUES 16384
 #define AO_MAX_TILES (AO_VALUES / 32 / AG_KEYS)

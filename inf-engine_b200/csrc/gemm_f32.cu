@@ -8,16 +8,16 @@
 // Even and odd k are the two lanes of fma.rn.f32x2 (two IEEE float32 products a lane pair and instruction): neighbouring k lie
 // side by side in memory, so operands need neither a transpose nor a broadcast.
 //
-// stream: up to 16 rows.  The product is a read of W (4 bytes a weight): HBM bounds it.  (A tile kernel reads it at 3 % of
-//   HBM: tiles of 64 rows for 4, loads of 4 bytes, blocks that walk all of K alone.)  Warp w of a block or cluster owns run w
+// stream: up to 16 rows.  The product is a read of W (4 bytes a weight): HBM bounds it.  (A tile kernel reads it at 6 to
+//   14 % of HBM: tiles of 64 rows for 4, loads of 4 bytes, blocks that walk all of K alone.)  Warp w of a block or cluster owns run w
 //   of K and streams its slice of 32 or 64 weight rows (and of the few activation rows, which come from L2) through a ring
 //   of its own, 16 bytes a lane and copy; no barrier but one at the end of a group of rows.
-// tile: more rows.  64 x 128 (or 32 x 128) outputs a block, 8 x 4 (4 x 4) a thread; FFMA bounds it (300 rows: 588 GFLOP for
-//   a 1.2 G-weight model, 7.9 ms at 74 TFLOP/s).  Where the tiles alone leave SMs idle, the eight runs of K
+// tile: more rows.  64 x 128 (or 32 x 128) outputs a block, 8 x 8 (4 x 8) a thread; FFMA bounds it (300 rows: 588 GFLOP for
+//   a model whose layers hold 0.97 G weights, 7.9 ms at 74 TFLOP/s).  Where the tiles alone leave SMs idle, the eight runs of K
 //   go to the eight blocks of a cluster, which add up through distributed shared memory in the same order.
 //
-// Measured on B200, us of a product, before (gemm_simt.cu's tile kernel) and now.  4 rows of 16,384 x 2,048: 460 and 30 (4.4
-// TB/s), 128,256 x 2,048: 3,000 and 195 (5.4 TB/s).  300 rows of 16,384 x 2,048: 1,350 and 575 (35 TFLOP/s).  What holds the
+// Measured on B200, us of a product, before (gemm_simt.cu's tile kernel) and now.  4 rows of 16,384 x 2,048: 325 and 30 (4.4
+// TB/s), 128,256 x 2,048: 1,187 and 195 (5.4 TB/s).  300 rows of 16,384 x 2,048: 882 and 581 (35 TFLOP/s).  What holds the
 // tile kernel at half of the FFMA rate: two warps a scheduler (128 sums a thread), which barriers and waits leave idle.
 #include "common.cuh"
 
@@ -385,7 +385,7 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
   const long long tiles = (long long)((M + bm - 1) / bm) * ((N + GF_BN - 1) / GF_BN);
   if (tiles * GF_PARTS > 0x7fffffffLL) return IE_BAD_SIZE;
   // Two blocks an SM: below four tiles an SM the last round of tiles weighs too much, and the runs of K are spread instead
-  // (640 tiles of 300 rows x 16,384: spread 591 us, not 575; 80 tiles of 300 x 2,048 leave half the SMs idle unless spread)
+  // (640 tiles of 300 rows x 16,384: spread 591 us against 575; 80 tiles of 300 x 2,048 leave half the SMs idle unless spread)
   const bool split = tiles < 4LL * n_sms;
   if (low) return split ? launch_tile<4, true>(p, (int)tiles, stream) : launch_tile<4, false>(p, (int)tiles, stream);
   return split ? launch_tile<8, true>(p, (int)tiles, stream) : launch_tile<8, false>(p, (int)tiles, stream);

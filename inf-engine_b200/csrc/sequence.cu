@@ -52,7 +52,7 @@ __global__ void outnorm_accumulate_kernel(float* __restrict__ residual, const TY
 }
 
 // Rows on 16 bytes, up to 8,192 wide: a thread keeps 8 columns at a time in registers, all loads 16 bytes a lane and in flight together
-// (element by element a row is three trips to memory, one after the other: 2,048 rows of 2,048 took 17.7 us, 8.1 here; with the mixture's sum before it 26.2, 11.1 here).
+// (element by element a row is three trips to memory, one after the other: 2,048 rows of 2,048 took 13.1 us, 9.1 here; with the mixture's sum before it 33.6 in two kernels, 11.4 here).
 // COMBINE: the row is not there yet; it is the weighted sum of a mixture's chosen experts plus the shared expert's,
 // sum over r of weights[t, r] * y[t * top + r] (r upward) + gate[t] * shared[t], which then never goes to memory.
 // THREADS: a warp for rows of up to 256 numbers (2,048 rows of 64: 2.7 us element by element, 4.7 with 256 threads of which
@@ -368,7 +368,7 @@ causal_conv_kernel(const TA* __restrict__ x, int x_stride, const TW* __restrict_
 
 // bfloat16 rows on 16 bytes, filters of up to four taps: a thread takes 8 channels and 8 tokens in a row and keeps the inputs of the
 // filter's length in registers, so a row is read once, 16 bytes a lane (the kernel above reads two bytes a lane and every row
-// `taps` times).  The caller says where this pays (`in_runs`: short requests leave most of a run empty).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 79 us, 23 so.
+// `taps` times).  The caller says where this pays (`in_runs`: short requests leave most of a run empty).  The same products in the same order: the same bits.  2,048 tokens of 3,072 channels: 68 us, 23 so.
 #define CV_CH 8
 #define CV_RUN 8
 template <typename TW, int TAPS>
@@ -576,11 +576,11 @@ linear_recurrence_kernel(const TA* __restrict__ u, int u_stride, const TA* __res
   if (write_state) state[(size_t)slot * width + c] = S;
 }
 
-// Many tokens: the chain above walks a request's tokens in one thread a channel (2,048 tokens of 2,048 channels: 1,042 us, 16
+// Many tokens: the chain above walks a request's tokens in one thread a channel (2,048 tokens of 2,048 channels: 16
 // blocks, each token's exponentials in the chain).  Here a block takes 16 channels and LS_SLICES runs of LS_TOK tokens; a
 // thread forms the decays and inputs of its run, runs it from a state of zero, and the runs' (sum of log a, end state)
 // pairs are put together by a scan in shared memory; then the run goes again from the state it really starts with.
-// 2,048 tokens of 2,048 channels: 860 us token after token, 47 so.
+// 2,048 tokens of 2,048 channels, launches one behind another: 805 us token after token, 47 so.
 #define LS_CH 16
 #define LS_SLICES 64
 #define LS_TOK 8

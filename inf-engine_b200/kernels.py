@@ -377,7 +377,6 @@ def attention_rows(q: torch.Tensor, out: torch.Tensor, kpool: torch.Tensor, vpoo
            f"attention_rows(head_dim={head_dim}, heads={n_heads}/{n_kv_heads})")
 
 
-# -------------------------------------------------------------------------- gemm
 def attention_ordered_rows(q: torch.Tensor, out: torch.Tensor, kpool: torch.Tensor, vpool: torch.Tensor, block_table: torch.Tensor,
                            q_start: torch.Tensor, ctx_before: torch.Tensor, n_requests: int, max_rows: int, n_heads: int,
                            n_kv_heads: int, head_dim: int, page_size: int, window: int | None, scale: float,
@@ -396,6 +395,7 @@ def attention_ordered_rows(q: torch.Tensor, out: torch.Tensor, kpool: torch.Tens
         f"attention_ordered_rows(head_dim={head_dim}, heads={n_heads}/{n_kv_heads})")
 
 
+# -------------------------------------------------------------------------- gemm
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     """out[M,N] = a[M,K] @ w[N,K]^T in float32 arithmetic."""
     m, k = a.shape

@@ -318,6 +318,8 @@ class PagedAttention:
         # requests at 300 keys: 134 us on the tile kernel, 21 so); the others split the keys over the block's warps
         newer = self.row_mode or self.keep_first or self.out_scale != 1.0
         n_small = ctx.n_requests if ctx.max_q_len * group <= 16 else ctx.keys_of_small_requests(group, 16)[0]
+        if not newer and not ordered_rows_pay(n_small, ctx.n_requests, s.head_dim, self.v_dim):
+            n_small = 0
         if n_small:
             if newer:
                 kernels.attention_rows(q, out, cache.k, cache.v, kvctx.block_table, ctx.q_start, ctx.ctx_before,
@@ -345,6 +347,14 @@ class PagedAttention:
                                   work_req, work_pair0, n_work, s.n_heads, s.n_kv_heads, s.head_dim,
                                   ctx.page_size, s.window, self.scale, bias, head_scale, self.v_dim, self.keep_first,
                                   self.out_scale)
+
+
+def ordered_rows_pay(n_small: int, n_requests: int, head_dim: int, v_dim: int) -> bool:
+    """Whether decode tokens of plain float32-arithmetic layers get a launch of their own (``attention_ordered_rows``).  Beside prompt
+    portions that launch also holds a block for every token of theirs, which only leaves; the rest of the step makes up for it
+    where the tile kernel moves 16 bytes at a time (a prompt of 300 beside two decode tokens, 32 heads of 64: 170 us in one
+    launch, 98 in two), not for other head sizes (4 heads of 20: 74 and 81)."""
+    return n_small > 0 and (n_small == n_requests or (head_dim % 8 == 0 and v_dim % 8 == 0))
 
 
 # fewer (token, head-in-group) rows than this in every request: the 64-row mma.sync tiles waste less

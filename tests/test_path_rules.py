@@ -15,3 +15,12 @@ def test_experts_through_the_ring(hidden, inter, blocks, ring):
                                              (4, 16, 2.1, 2.8), (16, 16, 2.2, 5.4), (16, 512, 36.7, 24.8), (17, 256, 15.7, 16.0)])
 def test_gate_products_of_a_few_rows(m, k, tiles, warps):
     assert kernels.diag_rows_pay(m, k) == (warps < tiles)
+
+
+# float32-arithmetic attention, us: (requests with few rows, requests, head size, one launch for all, two)
+@pytest.mark.parametrize("n_small,n_requests,hd,one,two", [(4, 4, 64, 134, 21), (2, 3, 64, 170, 98), (8, 9, 96, 3449, 1597), (2, 3, 20, 74, 81),
+                                                           (8, 9, 20, 487, 517), (4, 4, 20, 64, 15)])
+def test_a_launch_of_its_own_for_decode_tokens(n_small, n_requests, hd, one, two):
+    from inf_engine_b200.parts.attention import ordered_rows_pay
+    assert ordered_rows_pay(n_small, n_requests, hd, hd) == (two < one)
+    assert not ordered_rows_pay(0, n_requests, hd, hd)

@@ -481,10 +481,11 @@ def outnorm_accumulate(residual: torch.Tensor, y: torch.Tensor, gain: torch.Tens
                                         _stream()), "outnorm_accumulate")
 
 
-def moe_combine_outnorm_supports(residual: torch.Tensor, shared_out: torch.Tensor | None) -> bool:
+def moe_combine_outnorm_supports(residual: torch.Tensor, shared_out: torch.Tensor | None, gain: torch.Tensor,
+                                 next_in: torch.Tensor | None = None) -> bool:
     d = residual.shape[1]
-    return (d % 8 == 0 and d <= 8192 and residual.data_ptr() % 16 == 0
-            and (shared_out is None or (shared_out.stride(0) % 8 == 0 and shared_out.data_ptr() % 16 == 0)))
+    return (d % 8 == 0 and d <= 8192 and residual.data_ptr() % 16 == 0 and gain.data_ptr() % 16 == 0
+            and (next_in is None or next_in.data_ptr() % 16 == 0) and (shared_out is None or (shared_out.stride(0) % 8 == 0 and shared_out.data_ptr() % 16 == 0)))
 
 
 def moe_combine_outnorm(residual: torch.Tensor, y: torch.Tensor, weights: torch.Tensor, gate: torch.Tensor | None,

@@ -76,7 +76,7 @@ class RMSNorm:
     def accumulate_mixture(self, residual: torch.Tensor, parts, next_in: torch.Tensor | None = None) -> None:
         """``accumulate`` of a mixture of experts that is not summed up yet (``RoutedExperts.forward_parts``)."""
         y, weights, gate, shared = parts
-        if kernels.moe_combine_outnorm_supports(residual, shared):
+        if kernels.moe_combine_outnorm_supports(residual, shared, self.gain, next_in):
             kernels.moe_combine_outnorm(residual, y, weights, gate, shared, self.gain, self.eps, next_in)
             return
         out = self.rt.ws.take("moe_out", tuple(residual.shape), torch.float32)

@@ -176,3 +176,20 @@ def test_mixture_normed_into_the_stream(dtype, n, d, top, shared, gated):
     k.moe_combine(y, w, gate, sh, out)
     k.outnorm_accumulate(plain, out, gain, 1e-5)
     assert torch.equal(plain, got)
+
+
+@pytest.mark.parametrize("off", [0, 1])
+def test_a_gain_that_starts_off_16_bytes(off):
+    """A norm's gain may be any piece of a program's memory; the kernel with the mixture's sum in it wants 16-byte rows."""
+    from types import SimpleNamespace
+    from inf_engine_b200.parts.norms import RMSNorm
+    from inf_engine_b200.parts.runtime import Runtime
+    n, d, top = 3, 512, 2
+    flat = (1 + 0.1 * rnd(6, d + 8)).bfloat16()
+    norm = RMSNorm(SimpleNamespace(weight="w", eps=1e-5, size=d), {"w": flat[off:off + d]}, Runtime("cuda:0", torch.bfloat16))
+    y, w, res = rnd(1, n * top, d), rnd(2, n, top).abs(), rnd(3, n, d)
+    row = (w[:, :, None].double() * y.view(n, top, d).double()).sum(1)
+    want = res.double() + row / torch.sqrt((row * row).mean(-1, keepdim=True) + 1e-5) * norm.gain.double()
+    got = res.clone()
+    norm.accumulate_mixture(got, (y, w, None, None))
+    assert bool(((got.double() - want).abs() <= 3e-6 * (1 + want.abs())).all())

@@ -669,19 +669,18 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   const int lo_all = (min_first / DC_KT) * DC_KT;
 
   const int span = max_lim + 1 - lo_all;
-  const DecodeSplit own = decode_split(span, p.split_keys, (int)gridDim.x, p.spread != 0, DC_WARPS, DC_KT);
-  const int k_lo = lo_all + split * own.keys;
-  const int k_hi = min(k_lo + own.keys, max_lim + 1);
+  const int split_keys = decode_split_keys(span, p.split_keys, (int)gridDim.x, p.spread != 0, DC_WARPS, DC_KT);
+  const int k_lo = lo_all + split * split_keys;
+  const int k_hi = min(k_lo + split_keys, max_lim + 1);
   const bool has_work = k_lo <= max_lim && n_pairs > 0;
-  const int n_active_blocks = own.blocks;                     // blocks that hold at least one split: the first ones
   // A block without keys leaves at once and frees its slot.  It need not wait for the kernel ahead:
   // block 0 of every (request, kv head) always has keys and waits, so this kernel still ends after it.
   // (a request with more than 16 rows is not this kernel's: in a mixed step the prefill kernel takes it)
   if (n_pairs <= 0 || n_pairs > 16) return;                   // all blocks of this (request, kv head) alike
   // whether the blocks add up inside their cluster: the same answer in every block of the cluster, and every one
   // of them, with keys or without, then meets both cluster barriers below
-  const bool merge_in_cluster = p.cluster_merge != 0 && n_active_blocks > 1;
-  if ((int)blockIdx.x >= n_active_blocks) {
+  const bool merge_in_cluster = p.cluster_merge != 0 && span > DC_WARPS * split_keys;
+  if (blockIdx.x > 0 && (int)blockIdx.x * DC_WARPS * split_keys >= span) {
     if (merge_in_cluster) {
       cluster_barrier();
       cluster_barrier();
@@ -788,6 +787,7 @@ __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) att
   TRACE(5);                                                  // warp 0's tiles done, partial in shared memory
   __syncthreads();
   TRACE(6);                                                  // all warps of the block done
+  const int n_active_blocks = decode_split_blocks(span, split_keys, DC_WARPS);      // the first ones
   const int n_out = n_pairs * HD;
   const int blk = (int)blockIdx.x;
   for (int idx = threadIdx.x; idx < n_out; idx += DC_THREADS) {

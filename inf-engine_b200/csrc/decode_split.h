@@ -1,11 +1,6 @@
 // How one request's keys are cut in a decode attention launch (attention_mma.cu).
 #pragma once
 
-struct DecodeSplit {
-  int keys;       // keys of a warp, whole tiles
-  int blocks;     // blocks of the launch that hold some of the request's keys
-};
-
 // The launch gives every (request, kv head) `launch_blocks` blocks of `warps` warps, cut for the step's longest request:
 // `launch_keys` keys a warp, in tiles of `tile`.  A request spreads its `span` keys evenly over the warps of its blocks, at least 64
 // a warp (or the launch's cut, if that is shorter); with the launch's cut for all, a request of a quarter of the longest one's
@@ -16,11 +11,12 @@ struct DecodeSplit {
 // cut would fill: the others leave at once and make room (21 requests of 512 to 3,500 keys, heads of 64, two blocks each:
 // 33.3 us over all blocks, 24.9 so; with the launch's cut inside the blocks as well 26.3).
 #ifdef __CUDACC__
-__host__ __device__ __forceinline__
+#define IE_SPLIT_FN __host__ __device__ __forceinline__
 #else
-static inline
+#define IE_SPLIT_FN static inline
 #endif
-DecodeSplit decode_split(int span, int launch_keys, int launch_blocks, bool spread, const int warps, const int tile) {
+// Keys of a warp, whole tiles.
+IE_SPLIT_FN int decode_split_keys(int span, int launch_keys, int launch_blocks, bool spread, const int warps, const int tile) {
   const int least = launch_keys < 64 ? launch_keys : 64;
   int blocks = launch_blocks;
   if (launch_blocks > 1 && !spread) {
@@ -29,8 +25,10 @@ DecodeSplit decode_split(int span, int launch_keys, int launch_blocks, bool spre
   }
   const int even = blocks == 1 ? (span + warps - 1) / warps : (span + blocks * warps - 1) / (blocks * warps);
   const int whole = (even + tile - 1) / tile * tile;
-  DecodeSplit s;
-  s.keys = whole > least ? whole : least;
-  s.blocks = blocks == 1 ? 1 : (span + s.keys * warps - 1) / (s.keys * warps);      // (whole tiles may need fewer)
-  return s;
+  return whole > least ? whole : least;
+}
+
+// Blocks that hold some of the request's keys: the first ones (a block's own answer, block * warps * keys < span, needs no division).
+IE_SPLIT_FN int decode_split_blocks(int span, int keys, const int warps) {
+  return span <= keys * warps ? 1 : (span + keys * warps - 1) / (keys * warps);
 }

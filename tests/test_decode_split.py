@@ -10,8 +10,8 @@ HEADER = Path(__file__).resolve().parent.parent / "inf-engine_b200" / "csrc" / "
 SOURCE = """
 #include "decode_split.h"
 extern "C" void cut(int span, int launch_keys, int launch_blocks, int spread, int warps, int tile, int* out) {
-  const DecodeSplit s = decode_split(span, launch_keys, launch_blocks, spread != 0, warps, tile);
-  out[0] = s.keys; out[1] = s.blocks;
+  out[0] = decode_split_keys(span, launch_keys, launch_blocks, spread != 0, warps, tile);
+  out[1] = decode_split_blocks(span, out[0], warps);
 }
 """
 

@@ -101,6 +101,7 @@ struct TmaParams {
   const float* ssq_in;    // [SSQ_SLOT rows][ssq_blocks] the sums of the product ahead (PRENORMED)
   int ssq_blocks;
   float act_alpha, act_limit, act_offset, act_cubic;   // GLU
+  int pro, epi;           // products with activations in registers (their epilogue warp chooses as it runs)
 };
 
 // the gated activation of the GLU epilogue: g' sigmoid(alpha g' + cubic g'^3) (u' + offset), g' = min(g, limit) and u' = u
@@ -535,6 +536,318 @@ __device__ __forceinline__ void finish_units(const TmaParams& p, const BlockCtx&
   }
 }
 
+// ---------------------------------------------------------------- rings of warps
+// Plain or handed-over bfloat16 activations of a K of 1,024, 2,048, 3,072 or a multiple of 2,048 (what divides into the warps' stages)
+// take another form: every consumer warp streams its own columns of the weights through a ring of its own, 16 bytes a lane and copy, so no warp waits for another before the epilogue.
+// What bounded the shared ring was the bulk copies: an SM finishes one about every 90 clocks however short it is, so pieces of a
+// weight row of 2 KB just keep up with HBM, shorter ones do not, and rings that fit twice on an SM had no room for longer ones.
+// The warp multiplies the same columns of every unit, so its share of the activations is fetched once, straight into MMA
+// fragments (XC > 0: K = 256 XC), or, for a long K, a stage ahead (XC = 0: K a multiple of 2,048): nothing is staged and no
+// barrier comes between the kernel ahead and the first MMA.  Only the epilogue needs the 1/rms of a handed-over norm, so the
+// warps form it beside the first unit; the epilogue warp also asks for the residual before the sums are there.
+// Measured on B200, us of a layer's four products (qkv, output, gate/up, down) in a captured chain, 1, 8 and 16 rows, before (all
+// warps on one ring of bulk copies) and now: hidden 2,048 35.1, 37.3, 47.2 and 29.1, 31.1, 34.2 (18.6 of bytes); hidden
+// 3,072 51.1, 55.0, 73.9 and 42.1, 44.8, 48.9 (30.8).  Activations staged in shared memory took 1 to 1.9 us of every product
+// (8 rows; 3.3 at 16), the shared ring 0.44 us for 16 KB.
+constexpr int FLOW_THREADS = CONSUMER_THREADS + 32;        // + the epilogue warp
+template <int NT>
+struct FlowShape {                                         // a stage: 16 KB over the block
+  static constexpr int CHUNKS = 4 / NT;                    // of 32 k, a warp
+  static constexpr int K = 32 * CHUNKS, KS = K * CONSUMER_WARPS;
+  static constexpr int ROW_BYTES = 2 * K, STAGE_BYTES = 8 * NT * ROW_BYTES;
+  static constexpr int AHEAD = NT == 1 ? 2 : 4;            // buffers of activations of a long K
+};
+
+__device__ __forceinline__ void flow_copy16(uint32_t dst, const void* src, bool there, uint64_t pol) {
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void flow_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void flow_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <int NT, bool TWO, int XC, int STAGES>
+__device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* smem, float* red_mem, float* inv_rms) {
+  using F = FlowShape<NT>;
+  constexpr int UNIT_ROWS = 8 * NT, CHUNKS = F::CHUNKS, LANES = F::ROW_BYTES / 16, ROWS = 32 / LANES;
+  constexpr int XN = XC > 0 ? XC : F::AHEAD * CHUNKS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n_units = (p.N + UNIT_ROWS - 1) / UNIT_ROWS;
+  const int k_stages = XC > 0 ? XC / CHUNKS : p.K / F::KS;
+  float (*red)[CONSUMER_WARPS][4 * NT][32] = reinterpret_cast<float (*)[CONSUMER_WARPS][4 * NT][32]>(red_mem);
+  const uint32_t ring = smem_addr(smem) + warp * (STAGES * F::STAGE_BYTES);
+
+  // ---- weights: 16-byte pieces of odd rows change halves of 128 bytes, so that the fragments' reads (8 rows, 4 pieces) touch
+  // every bank once a quarter warp
+  const uint64_t pol = l2_evict_first_policy();
+  const int cr = lane / LANES, cc = lane % LANES;
+  const uint32_t c_dst = ring + cr * F::ROW_BYTES + ((cc ^ ((cr & 1) * 4)) << 4);
+  const int my_units = (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int total = my_units * k_stages;
+  int unit = blockIdx.x, ksi = 0, issued = 0, slot_in = 0;
+  auto copy = [&]() {
+    if (issued < total) {
+      const int n0 = unit * UNIT_ROWS + cr;
+      const bf16* src = p.W + (size_t)n0 * p.ldw + ksi * F::KS + warp * F::K + cc * 8;
+      const uint32_t dst = c_dst + slot_in * F::STAGE_BYTES;
+#pragma unroll
+      for (int i = 0; i < UNIT_ROWS / ROWS; ++i) {
+        const bool there = n0 + ROWS * i < p.N;
+        flow_copy16(dst + i * 512, there ? src + (size_t)(ROWS * i) * p.ldw : p.W, there, pol);
+      }
+      if (++ksi == k_stages) { ksi = 0; unit += gridDim.x; }
+    }
+    flow_commit();
+    ++issued;
+    if (++slot_in == STAGES) slot_in = 0;
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES; ++s) copy();
+
+  // ---- activations, and the 1/rms of rows warp and warp + 8
+  const bf16* const xa = (const bf16*)p.A + (size_t)(g < p.M ? g : 0) * p.lda + warp * F::K + t * 8;
+  const bf16* const xb = (const bf16*)p.A + (size_t)(g + 8 < p.M ? g + 8 : 0) * p.lda + warp * F::K + t * 8;
+  const bool va = g < p.M, vb = g + 8 < p.M;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 x0[XN], x1[TWO ? XN : 1];
+  auto fetch = [&](int to, int offset) {
+    x0[to] = va ? __ldcg(reinterpret_cast<const uint4*>(xa + offset)) : zero;
+    if (TWO) x1[to] = vb ? __ldcg(reinterpret_cast<const uint4*>(xb + offset)) : zero;
+  };
+  pdl_wait();
+  constexpr int FIRST = XC > 0 ? XC : (F::AHEAD - 1) * CHUNKS;
+#pragma unroll
+  for (int c = 0; c < FIRST; ++c) fetch(c, c / CHUNKS * F::KS + c % CHUNKS * 32);
+  float part[TWO ? 2 : 1];
+  if (p.pro == PRO_PRENORMED) {
+#pragma unroll
+    for (int h = 0; h < (TWO ? 2 : 1); ++h) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = warp + 8 * h < p.M && j * 32 + lane < p.ssq_blocks ? __ldcg(p.ssq_in + (size_t)(warp + 8 * h) * p.ssq_blocks + j * 32 + lane) : 0.f;
+      part[h] = v[0];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) part[h] += v[j];
+    }
+  }
+
+  int parity = 0, n_done = 0, slot = 0;
+  const uint32_t w_at = ring + g * F::ROW_BYTES, odd = (g & 1) * 4;
+  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+    // two accumulators per n-tile: the two MMAs of a chunk do not wait for each other
+    float acc[NT][2][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[nt][0][e] = acc[nt][1][e] = 0.f;
+    auto stage = [&](int x_at) {
+      flow_wait<STAGES - 1>();
+      __syncwarp();
+      const uint32_t wbase = w_at + slot * F::STAGE_BYTES;
+      uint4 w[CHUNKS][NT];
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) w[c][nt] = lds128(wbase + nt * 8 * F::ROW_BYTES + (((c * 4 + t) ^ odd) << 4));
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c) {
+        const uint4 a = x0[x_at + c], h = TWO ? x1[x_at + c] : zero;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          mma16816(acc[nt][0], a.x, h.x, a.y, h.y, w[c][nt].x, w[c][nt].y);
+          mma16816(acc[nt][1], a.z, h.z, a.w, h.w, w[c][nt].z, w[c][nt].w);
+        }
+      }
+      __syncwarp();                                          // every lane has read the slot
+      copy();
+      if (++slot == STAGES) slot = 0;
+    };
+    if (XC > 0) {
+#pragma unroll
+      for (int i = 0; i < (XC > 0 ? XC / CHUNKS : 1); ++i) stage(i * CHUNKS);
+    } else {
+      for (int i = 0; i < k_stages; i += F::AHEAD) {
+#pragma unroll
+        for (int j = 0; j < F::AHEAD; ++j) {
+          // the columns of AHEAD - 1 stages on (of the next unit, if this one ends: they are the same)
+          const int next = i + j + F::AHEAD - 1 < k_stages ? i + j + F::AHEAD - 1 : i + j + F::AHEAD - 1 - k_stages;
+#pragma unroll
+          for (int c = 0; c < CHUNKS; ++c) fetch((j + F::AHEAD - 1) % F::AHEAD * CHUNKS + c, next * F::KS + c * 32);
+          stage(j * CHUNKS);
+        }
+      }
+    }
+    if (n_done == 0 && p.pro == PRO_PRENORMED) {             // the epilogue warp reads them behind its first barrier
+#pragma unroll
+      for (int h = 0; h < (TWO ? 2 : 1); ++h) {
+        const float ssq = warp_sum(part[h]);
+        if (lane == 0) inv_rms[warp + 8 * h] = 1.f / sqrtf(ssq / (float)p.K + p.eps);
+      }
+    }
+    // this warp's partial sums -> red[parity]; the buffer was last used two units ago, and the epilogue warp has
+    // said when it had read it
+    if (n_done >= 2) named_sync(4 + parity);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) red[parity][warp][nt * 4 + e][lane] = acc[nt][0][e] + acc[nt][1][e];
+    named_arrive(2 + parity);
+    parity ^= 1;
+    ++n_done;
+  }
+  flow_wait<0>();
+}
+
+// The epilogue warp of those products: as finish_units, with prologue and epilogue chosen as it runs.
+template <int NT>
+__device__ __forceinline__ void finish_flow(const TmaParams& p, float* red_mem, const float* inv_rms) {
+  constexpr int UNIT_ROWS = 8 * NT;
+  const int lane = threadIdx.x & 31, gg = lane >> 2, tt = lane & 3, epi = p.epi;
+  const int n_units = (p.N + UNIT_ROWS - 1) / UNIT_ROWS;
+  float (*red)[CONSUMER_WARPS][4 * NT][32] = reinterpret_cast<float (*)[CONSUMER_WARPS][4 * NT][32]>(red_mem);
+  const bool adds = epi == EPI_RESIDUAL || epi == EPI_RESIDUAL_NORMOUT;
+  auto gain_at = [&](int n) {
+    return p.gain_next_is_f32 ? ((const float*)p.gain_next)[n] : __bfloat162float(((const bf16*)p.gain_next)[n]);
+  };
+  pdl_wait();                                                // nothing is written before the kernel ahead has finished
+  float squares[2] = {0.f, 0.f};       // RESIDUAL_NORMOUT: of the new residual values of rows gg and gg + 8
+  int parity = 0;
+  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+    // what the sums are added to is asked for before they are there
+    float old[NT][2][2], gain[NT][2];
+    if (adds) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int n = u * UNIT_ROWS + nt * 8 + tt * 2;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            old[nt][h][e] = gg + h * 8 < p.M && n + e < p.N ? __ldcg((const float*)p.C + (size_t)(gg + h * 8) * p.ldc + n + e) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) gain[nt][e] = epi == EPI_RESIDUAL_NORMOUT && n + e < p.N ? gain_at(n + e) : 0.f;
+      }
+    }
+    named_sync(2 + parity);                                  // every consumer warp has left its sums
+    {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = gg + h * 8, n = u * UNIT_ROWS + nt * 8 + tt * 2;
+          if (h * 8 >= p.M) continue;
+          float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+          for (int w = 0; w < CONSUMER_WARPS; ++w) {
+            v0 += red[parity][w][nt * 4 + h * 2][lane];
+            v1 += red[parity][w][nt * 4 + h * 2 + 1][lane];
+          }
+          if (m >= p.M || n >= p.N) continue;
+          if (p.pro == PRO_PRENORMED) {
+            v0 *= inv_rms[m];
+            v1 *= inv_rms[m];
+          }
+          const bool has1 = n + 1 < p.N;
+          if (adds) {
+            float* c = (float*)p.C + (size_t)m * p.ldc + n;
+            const float r0 = old[nt][h][0] + v0, r1 = has1 ? old[nt][h][1] + v1 : 0.f;
+            c[0] = r0;
+            if (has1) c[1] = r1;
+            if (epi == EPI_RESIDUAL_NORMOUT) {
+              squares[h] += r0 * r0 + r1 * r1;
+              bf16* xg = p.xg_out + (size_t)m * p.ld_xg + n;
+              if (has1 && ((((uintptr_t)xg) & 3) == 0)) *reinterpret_cast<uint32_t*>(xg) = pack2(r0 * gain[nt][0], r1 * gain[nt][1]);
+              else { xg[0] = __float2bfloat16_rn(r0 * gain[nt][0]); if (has1) xg[1] = __float2bfloat16_rn(r1 * gain[nt][1]); }
+            }
+          } else if (epi == EPI_F32) {
+            float* c = (float*)p.C + (size_t)m * p.ldc + n;
+            c[0] = v0;
+            if (has1) c[1] = v1;
+          } else if (epi == EPI_GLU) {
+            ((bf16*)p.C)[(size_t)m * p.ldc + (n >> 1)] = __float2bfloat16_rn(stream_glu(p, v0, v1));
+          } else if (epi == EPI_SILU_MUL) {
+            const float sg = 1.f / (1.f + expf(-v0));
+            ((bf16*)p.C)[(size_t)m * p.ldc + (n >> 1)] = __float2bfloat16_rn((v0 * sg) * v1);
+          } else {
+            if (epi == EPI_RELU2) {
+              v0 = stream_relu2(v0);
+              v1 = stream_relu2(v1);
+            }
+            bf16* c = (bf16*)p.C + (size_t)m * p.ldc + n;
+            if (has1 && ((((uintptr_t)c) & 3) == 0)) *reinterpret_cast<uint32_t*>(c) = pack2(v0, v1);
+            else { c[0] = __float2bfloat16_rn(v0); if (has1) c[1] = __float2bfloat16_rn(v1); }
+          }
+        }
+      }
+    }
+    // the consumers write this buffer again for the unit after the next: tell them that it has been read
+    if (u + 2 * (int)gridDim.x < n_units) named_arrive(4 + parity);
+    parity ^= 1;
+  }
+  if (epi == EPI_RESIDUAL_NORMOUT) {
+    // the block's sums of squares, row by row, in a fixed order: this lane's units and n-tiles in turn, then the four
+    // lanes of a row's quad
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      squares[h] += __shfl_xor_sync(0xffffffffu, squares[h], 1);
+      squares[h] += __shfl_xor_sync(0xffffffffu, squares[h], 2);
+      if (tt == 0) {
+        p.ssq_out[(size_t)(gg + 8 * h) * p.ssq_blocks + blockIdx.x] = squares[h];
+        // the reader adds ssq_blocks entries up: those of blocks that this launch does not have are zero
+        if (blockIdx.x == 0)
+          for (int j = gridDim.x; j < p.ssq_blocks; ++j) p.ssq_out[(size_t)(gg + 8 * h) * p.ssq_blocks + j] = 0.f;
+      }
+    }
+  }
+}
+
+// What every product's block begins with: the ring's barriers, and what its roles share.
+template <int NT>
+__device__ __forceinline__ BlockCtx begin_block(const TmaParams& p, unsigned char* smem, unsigned long long* bars, float* red,
+                                                float* inv_rms, volatile int* failed) {
+  BlockCtx b;
+  b.smem = smem;
+  b.ring = smem_addr(smem);
+  b.slot_bytes = (uint32_t)(8 * NT) * ((uint32_t)p.ks * 2 + ROW_PAD);
+  b.x_off = p.n_stages * b.slot_bytes;
+  b.full0 = smem_addr(&bars[0]);
+  b.empty0 = smem_addr(&bars[MAX_STAGES]);
+  b.n_stages = p.n_stages;
+  b.red = red;
+  b.inv_rms = inv_rms;
+  b.failed = failed;
+  if (threadIdx.x == 0) {
+    *failed = 0;
+    for (int s = 0; s < p.n_stages; ++s) {
+      mbar_init(b.full0 + 8 * s, 1);
+      mbar_init(b.empty0 + 8 * s, CONSUMER_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  return b;
+}
+__device__ __forceinline__ void producer_role(const TmaParams& p, int nt, const BlockCtx& b, RingPos& pos, int lane) {
+  const bool ok = produce(p, nt, b, pos, lane);
+  if (!ok && lane == 0) {
+    atomicExch(&g_stream_error, 1);
+    *b.failed = 1;
+    // copies already issued land in this block's shared memory: stay a bounded while before leaving
+    for (int i = 0; i < 4096; ++i) __nanosleep(64);
+  }
+  pdl_wait();
+}
+
+template <int NT, bool TWO, int XC, int STAGES>
+__global__ void __launch_bounds__(FLOW_THREADS, 1) gemm_stream_flow_kernel(TmaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float red[2][CONSUMER_WARPS][4 * NT][32];
+  __shared__ float inv_rms[16];
+  pdl_trigger();
+  if ((threadIdx.x >> 5) == CONSUMER_WARPS) finish_flow<NT>(p, &red[0][0][0][0], inv_rms);
+  else consume_flow<NT, TWO, XC, STAGES>(p, smem, &red[0][0][0][0], inv_rms);
+}
+
 // One product per launch.
 template <int NT, int PRO, int EPI, bool XS>
 // Units of 8 rows (short products: qkv, output) keep within 112 registers, so that the kernel behind them in
@@ -549,37 +862,11 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 2 : 1) gemm_stream_tma_kern
   pdl_trigger();
   TRACE_BEGIN();
   TRACE(0);                                                  // entry
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  BlockCtx b;
-  b.smem = smem;
-  b.ring = smem_addr(smem);
-  b.slot_bytes = (uint32_t)(8 * NT) * ((uint32_t)p.ks * 2 + ROW_PAD);
-  b.x_off = p.n_stages * b.slot_bytes;
-  b.full0 = smem_addr(&bars[0]);
-  b.empty0 = smem_addr(&bars[MAX_STAGES]);
-  b.n_stages = p.n_stages;
-  b.red = &red[0][0][0][0];
-  b.inv_rms = inv_rms;
-  b.failed = &failed;
-  if (tid == 0) {
-    failed = 0;
-    for (int s = 0; s < p.n_stages; ++s) {
-      mbar_init(b.full0 + 8 * s, 1);
-      mbar_init(b.empty0 + 8 * s, CONSUMER_WARPS);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const BlockCtx b = begin_block<NT>(p, smem, bars, &red[0][0][0][0], inv_rms, &failed);
   RingPos pos = {0, 0};
   if (warp == CONSUMER_WARPS) {
-    const bool ok = produce(p, NT, b, pos, lane);
-    if (!ok && lane == 0) {
-      atomicExch(&g_stream_error, 1);
-      failed = 1;
-      // copies already issued land in this block's shared memory: stay a bounded while before leaving
-      for (int i = 0; i < 4096; ++i) __nanosleep(64);
-    }
-    pdl_wait();
+    producer_role(p, NT, b, pos, lane);
     return;
   }
   if (warp == CONSUMER_WARPS + 1) {
@@ -776,6 +1063,29 @@ int launch_ring(const GroupedParams& p, int n_sms, size_t smem, cudaStream_t str
   return launch_k(moe_ring_kernel<NT, EPI>, n_sms, THREADS, smem, stream, p);
 }
 
+// Products in rings of warps
+template <int NT, bool TWO, int XC>
+int launch_flow_as(const TmaParams& p, int n_sms, cudaStream_t stream) {
+  // Rings of 96 KB, 128 KB for a long K (44.8 us a layer of hidden 3,072 against 45.2; 64 KB: 46.3), and more shared memory than
+  // two blocks of an SM can have.  Blocks of the kernel behind would else take the places that blocks of this one leave early, two on one SM
+  // while others have none, and the slowest SM decides: 38.7 us with 90 KB a block where 120 KB take 31.1.
+  constexpr int STAGES = XC == 0 ? 8 : 6, smem = STAGES == 6 ? 120 * 1024 : STAGES * 16 * 1024;
+  static OncePerDevice once;
+  const int ready = once([] {
+    return (int)cudaFuncSetAttribute(gemm_stream_flow_kernel<NT, TWO, XC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (ready) return ready;
+  const int n_units = (p.N + 8 * NT - 1) / (8 * NT);
+  return launch_k(gemm_stream_flow_kernel<NT, TWO, XC, STAGES>, n_units < n_sms ? n_units : n_sms, FLOW_THREADS, smem, stream, p);
+}
+template <int NT, bool TWO>
+int launch_flow(const TmaParams& p, int n_sms, cudaStream_t stream) {
+  if (p.K == 1024) return launch_flow_as<NT, TWO, 4>(p, n_sms, stream);
+  if (p.K == 2048) return launch_flow_as<NT, TWO, 8>(p, n_sms, stream);
+  if (p.K == 3072) return launch_flow_as<NT, TWO, 12>(p, n_sms, stream);
+  return launch_flow_as<NT, TWO, 0>(p, n_sms, stream);
+}
+
 template <int NT, int PRO, int EPI, bool XS>
 int launch_xs(const TmaParams& p, int n_sms, size_t smem, cudaStream_t stream) {
   static bool attr = false;
@@ -864,6 +1174,13 @@ extern "C" int ie_gemm_stream_tma(const void* A, const void* W, void* C, const v
       (!xg || !gain_next || !ssq || ssq_blocks < n_sms || (ld_xg & 1) || (((uintptr_t)xg | (uintptr_t)ssq) & 3)))
     return IE_BAD_SIZE;
   if (pro == PRO_PRENORMED && (!ssq || ssq_blocks <= 0 || ssq_blocks > 256)) return IE_BAD_SIZE;
+  p.pro = pro; p.epi = epi;
+  if (pro != PRO_NORM && (K == 1024 || K == 2048 || K == 3072 || K % 2048 == 0)) {
+    // as below: units of 16 rows where every SM still gets several, or, for a long K, about one
+    const bool wide = N >= 16 * 4 * n_sms || (K > 3072 && (N + 15) / 16 >= (n_sms * 3) / 4);
+    if (M > 8) return wide ? launch_flow<2, true>(p, n_sms, stream) : launch_flow<1, true>(p, n_sms, stream);
+    return wide ? launch_flow<2, false>(p, n_sms, stream) : launch_flow<1, false>(p, n_sms, stream);
+  }
   // units of 16 rows when that still gives every SM several units; a stage is 8 KB..16 KB per 8 rows
   p.x_rows = M > 8 ? 16 : 8;
   size_t x_bytes = (size_t)p.x_rows * ((size_t)K * 2 + ROW_PAD);

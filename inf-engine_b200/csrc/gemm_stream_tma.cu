@@ -1148,6 +1148,13 @@ extern "C" int ie_gemm_stream_trace_read(unsigned long long* out, int max_launch
 }
 #endif
 
+// Which epilogues a prologue has, whatever the form of the kernel.  A norm that is taken and one that is handed over do not meet in
+// one launch: both go by `xg` and `ssq`, and a block would write rows that others still read.
+static bool pair_is_taken(int pro, int epi) {
+  if (pro == PRO_PLAIN) return epi >= EPI_BF16 && epi <= EPI_GLU;
+  return (pro == PRO_NORM || pro == PRO_PRENORMED) && (epi == EPI_BF16 || epi == EPI_F32 || epi == EPI_SILU_MUL);
+}
+
 // pro 2 (PRENORMED): A is the bfloat16 [M, lda] that the product ahead wrote (its xg), ssq its sums of squares
 //   ([ssq_blocks, 16] float32), eps the norm's; gain unused.
 // epi 4 (RESIDUAL_NORMOUT): C float32 += product, and for the norm that comes next: xg [M, ld_xg] = bfloat16(C * gain_next)
@@ -1161,6 +1168,7 @@ extern "C" int ie_gemm_stream_tma(const void* A, const void* W, void* C, const v
   if (M <= 0 || N <= 0) return IE_OK;
   if (!ie_gemm_stream_tma_supports(M, N, K, pro) || (lda & 7) || (ldw & 7)) return IE_BAD_SIZE;
   if (((uintptr_t)A | (uintptr_t)W) & 15) return IE_BAD_ALIGN;
+  if (!pair_is_taken(pro, epi)) return IE_BAD_DTYPE;
   if ((epi == EPI_SILU_MUL || epi == EPI_GLU) && (N & 1)) return IE_BAD_SIZE;
   if (n_sms <= 0) return IE_BAD_SIZE;
   TmaParams p;

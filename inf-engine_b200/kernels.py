@@ -1518,12 +1518,15 @@ def gemm_stream(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, m: int, epi: 
     Two products can hand a norm over between them.  ``normout=(xg, gain_next, ssq)`` with epi "residual":
     besides adding into ``c`` the kernel writes ``xg`` = bfloat16(new c * gain_next) and, per block, the sums of
     squares of the new rows into ``ssq`` ([SSQ_SLOT rows, SMs] float32).  ``prenormed=(xg, ssq)`` with ``eps``: ``a`` is
-    ignored, the input is ``xg`` and the 1/rms comes from ``ssq``: RMSNorm without reading the residual again."""
+    ignored, the input is ``xg`` and the 1/rms comes from ``ssq``: RMSNorm without reading the residual again.  One product does
+    not do both: it would write the rows and sums that its own blocks still read."""
     n, k = w.shape
     assert w.dtype is torch.bfloat16 and w.stride(1) == 1 and a.stride(-1) == 1 and c.stride(-1) == 1
     lib = lib or stream_library()
     assert epi not in ("glu", "relu2") or (gain is None and prenormed is None)
     act = _act4(act)
+    if prenormed is not None and normout is not None:
+        raise KernelError("gemm_stream: prenormed and normout are not given to one product")
     if prenormed is not None or normout is not None:
         pro = 2 if prenormed is not None else 0
         xg, ssq = (prenormed if prenormed is not None else (normout[0], normout[2]))

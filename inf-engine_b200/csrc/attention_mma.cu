@@ -984,14 +984,12 @@ static int prefill_launch(const void* q, void* out, const void* kpool, const voi
   p.work_req = work_req;
   p.work_pair0 = work_pair0;
   const int smem = 2 * PF_STAGE_BYTES;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attention_prefill_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  const int ready = once([smem] {
+    const cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attention_prefill_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (ready) return ready;
   if (rows == 128) return launch_k(attention_prefill_kernel<8>, dim3(n_work, n_kv_heads), 256, smem, stream, p);
   return launch_k(attention_prefill_kernel<4>, dim3(n_work, n_kv_heads), 128, smem, stream, p);
 }
@@ -1058,12 +1056,9 @@ static int decode_launch(MmaAttnParams& p, float* scratch, int n_requests, int n
   p.part_o = scratch + IE_DECODE_TICKET_WORDS;
   p.part_ml = p.part_o + (size_t)n_tokens * n_heads * p.n_blocks * HD;
   const int smem = DC_SMEM_BYTES;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  const int ready = once([smem] { return cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  if (ready) return ready;
   // 2 to 8 blocks per (request, kv head): one cluster along x (-DIE_DC_NO_CLUSTER=1 builds the ticket path only),
   // but only while the whole launch has a place on the SMs at once.  A cluster starts when all its blocks find room
   // in one processing cluster at the same moment, and its blocks without keys stay until the others are done; in a

@@ -765,12 +765,11 @@ template <int HD, int KT, int STAGES, int PBUF, int SBUF, int MODE = 0>
 static int fa_launch(const CUtensorMap& mk, const CUtensorMap& mv, const FaParams& p, int n_work, int n_kv_heads,
                      cudaStream_t stream) {
   const size_t smem = Geo<HD, KT, STAGES, PBUF, SBUF>::TILES_BYTES + 128;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, KT, STAGES, PBUF, SBUF, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    attr = true;
-  }
+  static OncePerDevice once;
+  const int ready = once([smem] {
+    return cudaFuncSetAttribute(attention_tcgen05_kernel<HD, KT, STAGES, PBUF, SBUF, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (ready) return ready;
   return launch_k(attention_tcgen05_kernel<HD, KT, STAGES, PBUF, SBUF, MODE>, dim3((unsigned)((long long)n_work * n_kv_heads)), FA_THREADS, smem,
                   stream, mk, mv, p);
 }

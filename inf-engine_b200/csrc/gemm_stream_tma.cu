@@ -1088,13 +1088,11 @@ int launch_flow(const TmaParams& p, int n_sms, cudaStream_t stream) {
 
 template <int NT, int PRO, int EPI, bool XS>
 int launch_xs(const TmaParams& p, int n_sms, size_t smem, cudaStream_t stream) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_stream_tma_kernel<NT, PRO, EPI, XS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    attr = true;
-  }
+  static OncePerDevice once;
+  const int ready = once([] {
+    return cudaFuncSetAttribute(gemm_stream_tma_kernel<NT, PRO, EPI, XS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024);
+  });
+  if (ready) return ready;
   const int n_units = (p.N + 8 * NT - 1) / (8 * NT);
   const int grid = n_units < n_sms ? n_units : n_sms;
   return launch_k(gemm_stream_tma_kernel<NT, PRO, EPI, XS>, grid, THREADS, smem, stream, p);

@@ -512,12 +512,11 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, TcParams p, i
   if (n_stages > 8) n_stages = 8;
   p.n_stages = n_stages;
   const size_t smem = (size_t)n_stages * stage + 1024 + 4 * TC_STAGE_BYTES;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, GROUPED, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    attr = true;
-  }
+  static OncePerDevice once;
+  const int ready = once([smem] {
+    return cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, GROUPED, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (ready) return ready;
   const int tiles = (GROUPED ? p.max_tiles : (p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   const int grid = tiles < n_sms ? tiles : n_sms;
   return launch_k(gemm_tcgen05_kernel<BN, GROUPED, DIAG>, grid, TC_THREADS, smem, stream, ma, mw, p);

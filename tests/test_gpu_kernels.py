@@ -175,7 +175,8 @@ def test_gemm_stream_plain_and_fused(M, N, K):
 @pytest.mark.parametrize("M", [1, 5, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(389, 256), (1000, 768), (2050, 2048), (776, 3072), (520, 8192)])
 def test_gemm_stream_bulk_copy_kernel(M, N, K):
-    """The persistent kernel (weights by cp.async.bulk through a shared-memory ring), default for K % 256 == 0."""
+    """The persistent kernel, default for K % 256 == 0: weights by cp.async.bulk through a ring of the block (256 and 768 here, and every
+    norm in the prologue), or through rings of the warps (2,048, 3,072 and 8,192 without one)."""
     from inf_engine_b200 import kernels
     lib = kernels.stream_library()
     assert lib.ie_gemm_stream_tma_supports(M, N, K, 0)

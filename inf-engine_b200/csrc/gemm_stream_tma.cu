@@ -437,76 +437,94 @@ __device__ __forceinline__ void consume(const TmaParams& p, const BlockCtx& b, R
 }
 
 // ------------------------------------------------------------- epilogue (one warp)
+// Two neighbouring outputs (row, n), (row, n + 1) of an epilogue that stores; the second only with has1.
+template <int EPI, typename P>
+__device__ __forceinline__ void store_pair(const P& p, int row, int n, bool has1, float v0, float v1) {
+  if (EPI == EPI_F32) {
+    float* c = (float*)p.C + (size_t)row * p.ldc + n;
+    c[0] = v0;
+    if (has1) c[1] = v1;
+  } else if (EPI == EPI_GLU) {
+    ((bf16*)p.C)[(size_t)row * p.ldc + (n >> 1)] = __float2bfloat16_rn(stream_glu(p, v0, v1));
+  } else if (EPI == EPI_SILU_MUL) {
+    const float sg = 1.f / (1.f + expf(-v0));
+    ((bf16*)p.C)[(size_t)row * p.ldc + (n >> 1)] = __float2bfloat16_rn((v0 * sg) * v1);
+  } else {
+    if (EPI == EPI_RELU2) {
+      v0 = stream_relu2(v0);
+      v1 = stream_relu2(v1);
+    }
+    bf16* c = (bf16*)p.C + (size_t)row * p.ldc + n;
+    if (has1 && ((((uintptr_t)c) & 3) == 0)) *reinterpret_cast<uint32_t*>(c) = pack2(v0, v1);
+    else { c[0] = __float2bfloat16_rn(v0); if (has1) c[1] = __float2bfloat16_rn(v1); }
+  }
+}
+
 // Lane ln holds, per n-tile nt and half h, the two neighbouring outputs (m = ln / 4 + 8 h, n = unit + 8 nt + 2 (ln % 4)):
 // the layout of the MMA's accumulator, so the sums are read from red[] as the consumers wrote them.
-template <int NT, int PRO, int EPI>
-__device__ __forceinline__ void finish_units(const TmaParams& p, const BlockCtx& b, bool first) {
+// `failed`: the bulk copies' word (null for the rings of warps, which wait for nothing that can fail to come).
+template <int NT, int EPI>
+__device__ __forceinline__ void finish_units(const TmaParams& p, float* red_mem, const float* inv_rms, const volatile int* failed) {
   constexpr int UNIT_ROWS = 8 * NT;
-  const int lane = threadIdx.x & 31;
+  constexpr bool ADDS = EPI == EPI_RESIDUAL || EPI == EPI_RESIDUAL_NORMOUT;
+  const int lane = threadIdx.x & 31, gg = lane >> 2, tt = lane & 3;
   const int n_units = (p.N + UNIT_ROWS - 1) / UNIT_ROWS;
-  volatile int& failed = *b.failed;
-  const float* const inv_rms = b.inv_rms;
-  float (*red)[CONSUMER_WARPS][4 * NT][32] = reinterpret_cast<float (*)[CONSUMER_WARPS][4 * NT][32]>(b.red);
-  if (first) pdl_wait();                                     // nothing is written before the kernel ahead has finished
-  handover_sync();                                           // inv_rms is there
-  const int gg = lane >> 2, tt = lane & 3;
-  float ssq_lo = 0.f, ssq_hi = 0.f;    // RESIDUAL_NORMOUT: squares of the new residual values of rows gg and gg + 8
+  float (*red)[CONSUMER_WARPS][4 * NT][32] = reinterpret_cast<float (*)[CONSUMER_WARPS][4 * NT][32]>(red_mem);
+  const bool scaled = p.pro != PRO_PLAIN;
+  auto gain_at = [&](int n) {
+    return p.gain_next_is_f32 ? ((const float*)p.gain_next)[n] : __bfloat162float(((const bf16*)p.gain_next)[n]);
+  };
+  float squares[2] = {0.f, 0.f};       // RESIDUAL_NORMOUT: of the new residual values of rows gg and gg + 8
   int parity = 0;
   for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-    named_sync(2 + parity);                                  // every consumer warp has left its sums
-    if (!failed) {
+    // what the sums are added to is asked for before they are there
+    float old[NT][2][2], gain[NT][2];
+    if (ADDS) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
+        const int n = u * UNIT_ROWS + nt * 8 + tt * 2;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int m = gg + h * 8;
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            old[nt][h][e] = gg + h * 8 < p.M && n + e < p.N ? __ldcg((const float*)p.C + (size_t)(gg + h * 8) * p.ldc + n + e) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) gain[nt][e] = EPI == EPI_RESIDUAL_NORMOUT && n + e < p.N ? gain_at(n + e) : 0.f;
+      }
+    }
+    named_sync(2 + parity);                                  // every consumer warp has left its sums
+    if (!failed || !*failed) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h * 8 >= p.M) continue;
+        const int m = gg + h * 8;
+        const float scale = scaled && m < p.M ? inv_rms[m] : 1.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
           const int n = u * UNIT_ROWS + nt * 8 + tt * 2;
           float v0 = 0.f, v1 = 0.f;
 #pragma unroll
-          for (int w4 = 0; w4 < CONSUMER_WARPS; ++w4) {
-            v0 += red[parity][w4][nt * 4 + h * 2][lane];
-            v1 += red[parity][w4][nt * 4 + h * 2 + 1][lane];
+          for (int w = 0; w < CONSUMER_WARPS; ++w) {
+            v0 += red[parity][w][nt * 4 + h * 2][lane];
+            v1 += red[parity][w][nt * 4 + h * 2 + 1][lane];
           }
-          if (m < p.M && n < p.N) {
-            if (PRO != PRO_PLAIN) {
-              v0 *= inv_rms[m];
-              v1 *= inv_rms[m];
-            }
-            const bool has1 = n + 1 < p.N;
-            if (EPI == EPI_RELU2) {
-              v0 = stream_relu2(v0);
-              v1 = stream_relu2(v1);
-            }
-            if (EPI == EPI_BF16 || EPI == EPI_RELU2) {
-              bf16* c = (bf16*)p.C + (size_t)m * p.ldc + n;
-              if (has1 && ((((uintptr_t)c) & 3) == 0)) *reinterpret_cast<uint32_t*>(c) = pack2(v0, v1);
-              else { c[0] = __float2bfloat16_rn(v0); if (has1) c[1] = __float2bfloat16_rn(v1); }
-            } else if (EPI == EPI_F32) {
-              float* c = (float*)p.C + (size_t)m * p.ldc + n;
-              c[0] = v0;
-              if (has1) c[1] = v1;
-            } else if (EPI == EPI_RESIDUAL) {
-              float* c = (float*)p.C + (size_t)m * p.ldc + n;
-              c[0] += v0;
-              if (has1) c[1] += v1;
-            } else if (EPI == EPI_RESIDUAL_NORMOUT) {
-              float* c = (float*)p.C + (size_t)m * p.ldc + n;
-              const float r0 = c[0] + v0, r1 = has1 ? c[1] + v1 : 0.f;
-              c[0] = r0;
-              if (has1) c[1] = r1;
-              if (h == 0) ssq_lo += r0 * r0 + r1 * r1;
-              else ssq_hi += r0 * r0 + r1 * r1;
-              const float g0 = p.gain_next_is_f32 ? ((const float*)p.gain_next)[n] : __bfloat162float(((const bf16*)p.gain_next)[n]);
-              const float g1 = !has1 ? 0.f : (p.gain_next_is_f32 ? ((const float*)p.gain_next)[n + 1] : __bfloat162float(((const bf16*)p.gain_next)[n + 1]));
+          if (m >= p.M || n >= p.N) continue;
+          v0 *= scale;
+          v1 *= scale;
+          const bool has1 = n + 1 < p.N;
+          if (ADDS) {
+            float* c = (float*)p.C + (size_t)m * p.ldc + n;
+            const float r0 = old[nt][h][0] + v0, r1 = has1 ? old[nt][h][1] + v1 : 0.f;
+            c[0] = r0;
+            if (has1) c[1] = r1;
+            if (EPI == EPI_RESIDUAL_NORMOUT) {
+              squares[h] += r0 * r0 + r1 * r1;
               bf16* xg = p.xg_out + (size_t)m * p.ld_xg + n;
-              if (has1 && ((((uintptr_t)xg) & 3) == 0)) *reinterpret_cast<uint32_t*>(xg) = pack2(r0 * g0, r1 * g1);
-              else { xg[0] = __float2bfloat16_rn(r0 * g0); if (has1) xg[1] = __float2bfloat16_rn(r1 * g1); }
-            } else if (EPI == EPI_GLU) {
-              ((bf16*)p.C)[(size_t)m * p.ldc + (n >> 1)] = __float2bfloat16_rn(stream_glu(p, v0, v1));
-            } else {
-              const float sg = 1.f / (1.f + expf(-v0));
-              ((bf16*)p.C)[(size_t)m * p.ldc + (n >> 1)] = __float2bfloat16_rn((v0 * sg) * v1);
+              if (has1 && ((((uintptr_t)xg) & 3) == 0)) *reinterpret_cast<uint32_t*>(xg) = pack2(r0 * gain[nt][0], r1 * gain[nt][1]);
+              else { xg[0] = __float2bfloat16_rn(r0 * gain[nt][0]); if (has1) xg[1] = __float2bfloat16_rn(r1 * gain[nt][1]); }
             }
+          } else {
+            store_pair<EPI>(p, m, n, has1, v0, v1);
           }
         }
       }
@@ -518,20 +536,17 @@ __device__ __forceinline__ void finish_units(const TmaParams& p, const BlockCtx&
   if (EPI == EPI_RESIDUAL_NORMOUT) {
     // the block's sums of squares, row by row, in a fixed order: this lane's units and n-tiles in turn, then the four
     // lanes of a row's quad
-    ssq_lo += __shfl_xor_sync(0xffffffffu, ssq_lo, 1);
-    ssq_lo += __shfl_xor_sync(0xffffffffu, ssq_lo, 2);
-    ssq_hi += __shfl_xor_sync(0xffffffffu, ssq_hi, 1);
-    ssq_hi += __shfl_xor_sync(0xffffffffu, ssq_hi, 2);
-    if (tt == 0) {
-      // laid out [16 rows][ssq_blocks]: the reader's warp takes one row of it, contiguous
-      p.ssq_out[(size_t)gg * p.ssq_blocks + blockIdx.x] = ssq_lo;
-      p.ssq_out[(size_t)(gg + 8) * p.ssq_blocks + blockIdx.x] = ssq_hi;
-      // the reader adds ssq_blocks entries up: those of blocks that this launch does not have are zero
-      if (blockIdx.x == 0)
-        for (int j = gridDim.x; j < p.ssq_blocks; ++j) {
-          p.ssq_out[(size_t)gg * p.ssq_blocks + j] = 0.f;
-          p.ssq_out[(size_t)(gg + 8) * p.ssq_blocks + j] = 0.f;
-        }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      squares[h] += __shfl_xor_sync(0xffffffffu, squares[h], 1);
+      squares[h] += __shfl_xor_sync(0xffffffffu, squares[h], 2);
+      if (tt == 0) {
+        // laid out [16 rows][ssq_blocks]: the reader's warp takes one row of it, contiguous
+        p.ssq_out[(size_t)(gg + 8 * h) * p.ssq_blocks + blockIdx.x] = squares[h];
+        // the reader adds ssq_blocks entries up: those of blocks that this launch does not have are zero
+        if (blockIdx.x == 0)
+          for (int j = gridDim.x; j < p.ssq_blocks; ++j) p.ssq_out[(size_t)(gg + 8 * h) * p.ssq_blocks + j] = 0.f;
+      }
     }
   }
 }
@@ -698,154 +713,28 @@ __device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* 
   flow_wait<0>();
 }
 
-// The epilogue warp of those products: as finish_units, with prologue and epilogue chosen as it runs.
-template <int NT>
-__device__ __forceinline__ void finish_flow(const TmaParams& p, float* red_mem, const float* inv_rms) {
-  constexpr int UNIT_ROWS = 8 * NT;
-  const int lane = threadIdx.x & 31, gg = lane >> 2, tt = lane & 3, epi = p.epi;
-  const int n_units = (p.N + UNIT_ROWS - 1) / UNIT_ROWS;
-  float (*red)[CONSUMER_WARPS][4 * NT][32] = reinterpret_cast<float (*)[CONSUMER_WARPS][4 * NT][32]>(red_mem);
-  const bool adds = epi == EPI_RESIDUAL || epi == EPI_RESIDUAL_NORMOUT;
-  auto gain_at = [&](int n) {
-    return p.gain_next_is_f32 ? ((const float*)p.gain_next)[n] : __bfloat162float(((const bf16*)p.gain_next)[n]);
-  };
-  pdl_wait();                                                // nothing is written before the kernel ahead has finished
-  float squares[2] = {0.f, 0.f};       // RESIDUAL_NORMOUT: of the new residual values of rows gg and gg + 8
-  int parity = 0;
-  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-    // what the sums are added to is asked for before they are there
-    float old[NT][2][2], gain[NT][2];
-    if (adds) {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const int n = u * UNIT_ROWS + nt * 8 + tt * 2;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-            old[nt][h][e] = gg + h * 8 < p.M && n + e < p.N ? __ldcg((const float*)p.C + (size_t)(gg + h * 8) * p.ldc + n + e) : 0.f;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) gain[nt][e] = epi == EPI_RESIDUAL_NORMOUT && n + e < p.N ? gain_at(n + e) : 0.f;
-      }
-    }
-    named_sync(2 + parity);                                  // every consumer warp has left its sums
-    {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int m = gg + h * 8, n = u * UNIT_ROWS + nt * 8 + tt * 2;
-          if (h * 8 >= p.M) continue;
-          float v0 = 0.f, v1 = 0.f;
-#pragma unroll
-          for (int w = 0; w < CONSUMER_WARPS; ++w) {
-            v0 += red[parity][w][nt * 4 + h * 2][lane];
-            v1 += red[parity][w][nt * 4 + h * 2 + 1][lane];
-          }
-          if (m >= p.M || n >= p.N) continue;
-          if (p.pro == PRO_PRENORMED) {
-            v0 *= inv_rms[m];
-            v1 *= inv_rms[m];
-          }
-          const bool has1 = n + 1 < p.N;
-          if (adds) {
-            float* c = (float*)p.C + (size_t)m * p.ldc + n;
-            const float r0 = old[nt][h][0] + v0, r1 = has1 ? old[nt][h][1] + v1 : 0.f;
-            c[0] = r0;
-            if (has1) c[1] = r1;
-            if (epi == EPI_RESIDUAL_NORMOUT) {
-              squares[h] += r0 * r0 + r1 * r1;
-              bf16* xg = p.xg_out + (size_t)m * p.ld_xg + n;
-              if (has1 && ((((uintptr_t)xg) & 3) == 0)) *reinterpret_cast<uint32_t*>(xg) = pack2(r0 * gain[nt][0], r1 * gain[nt][1]);
-              else { xg[0] = __float2bfloat16_rn(r0 * gain[nt][0]); if (has1) xg[1] = __float2bfloat16_rn(r1 * gain[nt][1]); }
-            }
-          } else if (epi == EPI_F32) {
-            float* c = (float*)p.C + (size_t)m * p.ldc + n;
-            c[0] = v0;
-            if (has1) c[1] = v1;
-          } else if (epi == EPI_GLU) {
-            ((bf16*)p.C)[(size_t)m * p.ldc + (n >> 1)] = __float2bfloat16_rn(stream_glu(p, v0, v1));
-          } else if (epi == EPI_SILU_MUL) {
-            const float sg = 1.f / (1.f + expf(-v0));
-            ((bf16*)p.C)[(size_t)m * p.ldc + (n >> 1)] = __float2bfloat16_rn((v0 * sg) * v1);
-          } else {
-            if (epi == EPI_RELU2) {
-              v0 = stream_relu2(v0);
-              v1 = stream_relu2(v1);
-            }
-            bf16* c = (bf16*)p.C + (size_t)m * p.ldc + n;
-            if (has1 && ((((uintptr_t)c) & 3) == 0)) *reinterpret_cast<uint32_t*>(c) = pack2(v0, v1);
-            else { c[0] = __float2bfloat16_rn(v0); if (has1) c[1] = __float2bfloat16_rn(v1); }
-          }
-        }
-      }
-    }
-    // the consumers write this buffer again for the unit after the next: tell them that it has been read
-    if (u + 2 * (int)gridDim.x < n_units) named_arrive(4 + parity);
-    parity ^= 1;
-  }
-  if (epi == EPI_RESIDUAL_NORMOUT) {
-    // the block's sums of squares, row by row, in a fixed order: this lane's units and n-tiles in turn, then the four
-    // lanes of a row's quad
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      squares[h] += __shfl_xor_sync(0xffffffffu, squares[h], 1);
-      squares[h] += __shfl_xor_sync(0xffffffffu, squares[h], 2);
-      if (tt == 0) {
-        p.ssq_out[(size_t)(gg + 8 * h) * p.ssq_blocks + blockIdx.x] = squares[h];
-        // the reader adds ssq_blocks entries up: those of blocks that this launch does not have are zero
-        if (blockIdx.x == 0)
-          for (int j = gridDim.x; j < p.ssq_blocks; ++j) p.ssq_out[(size_t)(gg + 8 * h) * p.ssq_blocks + j] = 0.f;
-      }
-    }
-  }
-}
-
-// What every product's block begins with: the ring's barriers, and what its roles share.
-template <int NT>
-__device__ __forceinline__ BlockCtx begin_block(const TmaParams& p, unsigned char* smem, unsigned long long* bars, float* red,
-                                                float* inv_rms, volatile int* failed) {
-  BlockCtx b;
-  b.smem = smem;
-  b.ring = smem_addr(smem);
-  b.slot_bytes = (uint32_t)(8 * NT) * ((uint32_t)p.ks * 2 + ROW_PAD);
-  b.x_off = p.n_stages * b.slot_bytes;
-  b.full0 = smem_addr(&bars[0]);
-  b.empty0 = smem_addr(&bars[MAX_STAGES]);
-  b.n_stages = p.n_stages;
-  b.red = red;
-  b.inv_rms = inv_rms;
-  b.failed = failed;
-  if (threadIdx.x == 0) {
-    *failed = 0;
-    for (int s = 0; s < p.n_stages; ++s) {
-      mbar_init(b.full0 + 8 * s, 1);
-      mbar_init(b.empty0 + 8 * s, CONSUMER_WARPS);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  return b;
-}
-__device__ __forceinline__ void producer_role(const TmaParams& p, int nt, const BlockCtx& b, RingPos& pos, int lane) {
-  const bool ok = produce(p, nt, b, pos, lane);
-  if (!ok && lane == 0) {
-    atomicExch(&g_stream_error, 1);
-    *b.failed = 1;
-    // copies already issued land in this block's shared memory: stay a bounded while before leaving
-    for (int i = 0; i < 4096; ++i) __nanosleep(64);
-  }
-  pdl_wait();
-}
-
 template <int NT, bool TWO, int XC, int STAGES>
 __global__ void __launch_bounds__(FLOW_THREADS, 1) gemm_stream_flow_kernel(TmaParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ float red[2][CONSUMER_WARPS][4 * NT][32];
   __shared__ float inv_rms[16];
   pdl_trigger();
-  if ((threadIdx.x >> 5) == CONSUMER_WARPS) finish_flow<NT>(p, &red[0][0][0][0], inv_rms);
-  else consume_flow<NT, TWO, XC, STAGES>(p, smem, &red[0][0][0][0], inv_rms);
+  if ((threadIdx.x >> 5) < CONSUMER_WARPS) {
+    consume_flow<NT, TWO, XC, STAGES>(p, smem, &red[0][0][0][0], inv_rms);
+    return;
+  }
+  pdl_wait();                                                // nothing is written before the kernel ahead has finished
+  float* const sums = &red[0][0][0][0];
+  // chosen once a launch: chosen inside the loop of units it bounded a K of 1,024 (16,384 columns, 9 rows: 10.1 us, 7.7 so)
+  switch (p.epi) {
+    case EPI_BF16: finish_units<NT, EPI_BF16>(p, sums, inv_rms, nullptr); break;
+    case EPI_F32: finish_units<NT, EPI_F32>(p, sums, inv_rms, nullptr); break;
+    case EPI_RESIDUAL: finish_units<NT, EPI_RESIDUAL>(p, sums, inv_rms, nullptr); break;
+    case EPI_SILU_MUL: finish_units<NT, EPI_SILU_MUL>(p, sums, inv_rms, nullptr); break;
+    case EPI_RESIDUAL_NORMOUT: finish_units<NT, EPI_RESIDUAL_NORMOUT>(p, sums, inv_rms, nullptr); break;
+    case EPI_RELU2: finish_units<NT, EPI_RELU2>(p, sums, inv_rms, nullptr); break;
+    case EPI_GLU: finish_units<NT, EPI_GLU>(p, sums, inv_rms, nullptr); break;
+  }
 }
 
 // One product per launch.
@@ -863,14 +752,42 @@ __global__ void __launch_bounds__(THREADS, NT == 1 ? 2 : 1) gemm_stream_tma_kern
   TRACE_BEGIN();
   TRACE(0);                                                  // entry
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const BlockCtx b = begin_block<NT>(p, smem, bars, &red[0][0][0][0], inv_rms, &failed);
+  BlockCtx b;
+  b.smem = smem;
+  b.ring = smem_addr(smem);
+  b.slot_bytes = (uint32_t)(8 * NT) * ((uint32_t)p.ks * 2 + ROW_PAD);
+  b.x_off = p.n_stages * b.slot_bytes;
+  b.full0 = smem_addr(&bars[0]);
+  b.empty0 = smem_addr(&bars[MAX_STAGES]);
+  b.n_stages = p.n_stages;
+  b.red = &red[0][0][0][0];
+  b.inv_rms = inv_rms;
+  b.failed = &failed;
+  if (threadIdx.x == 0) {
+    failed = 0;
+    for (int s = 0; s < p.n_stages; ++s) {
+      mbar_init(b.full0 + 8 * s, 1);
+      mbar_init(b.empty0 + 8 * s, CONSUMER_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
   RingPos pos = {0, 0};
   if (warp == CONSUMER_WARPS) {
-    producer_role(p, NT, b, pos, lane);
+    const bool ok = produce(p, NT, b, pos, lane);
+    if (!ok && lane == 0) {
+      atomicExch(&g_stream_error, 1);
+      failed = 1;
+      // copies already issued land in this block's shared memory: stay a bounded while before leaving
+      for (int i = 0; i < 4096; ++i) __nanosleep(64);
+    }
+    pdl_wait();
     return;
   }
   if (warp == CONSUMER_WARPS + 1) {
-    finish_units<NT, PRO, EPI>(p, b, true);
+    pdl_wait();                                              // nothing is written before the kernel ahead has finished
+    handover_sync();                                         // inv_rms is there
+    finish_units<NT, EPI>(p, b.red, inv_rms, &failed);
     return;
   }
 #ifdef IE_STREAM_TRACE
@@ -972,20 +889,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
               v0 += red[parity][w][nt * 4 + h * 2][lane];
               v1 += red[parity][w][nt * 4 + h * 2 + 1][lane];
             }
-            if (at[h] >= 0 && n < p.N) {
-              const bool has1 = n + 1 < p.N;
-              if (EPI == EPI_GLU) {
-                ((bf16*)p.C)[(size_t)at[h] * p.ldc + (n >> 1)] = __float2bfloat16_rn(stream_glu(p, v0, v1));
-              } else if (EPI == EPI_RELU2) {
-                bf16* c = (bf16*)p.C + (size_t)at[h] * p.ldc + n;
-                c[0] = __float2bfloat16_rn(stream_relu2(v0));
-                if (has1) c[1] = __float2bfloat16_rn(stream_relu2(v1));
-              } else {
-                float* c = (float*)p.C + (size_t)at[h] * p.ldc + n;
-                c[0] = v0;
-                if (has1) c[1] = v1;
-              }
-            }
+            if (at[h] >= 0 && n < p.N) store_pair<EPI>(p, at[h], n, n + 1 < p.N, v0, v1);
           }
         }
       }

@@ -154,6 +154,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 // barrier 1: consumers and epilogue warp, once, when the activations are staged.  Barriers 2, 3 ("sums of unit are
 // in red[0], red[1]") and 4, 5 ("red[0], red[1] have been read"): the consumers arrive on the first pair without
 // waiting and the epilogue warp waits there; the other way round on the second pair.  So the consumers go on with the
@@ -552,29 +555,41 @@ __device__ __forceinline__ void finish_units(const TmaParams& p, float* red_mem,
 }
 
 // ---------------------------------------------------------------- rings of warps
-// Plain or handed-over bfloat16 activations of a K of 1,024, 2,048, 3,072 or a multiple of 2,048 (what divides into the warps' stages)
-// take another form: every consumer warp streams its own columns of the weights through a ring of its own, 16 bytes a lane and copy, so no warp waits for another before the epilogue.
-// What bounded the shared ring was the bulk copies: an SM finishes one about every 90 clocks however short it is, so pieces of a
+// Plain or handed-over bfloat16 activations of a K of 1,024, 2,048, 3,072 or a multiple of 2,048 take another form: every consumer
+// warp streams its own columns of the weights through a ring of its own, 16 bytes a lane and copy, so no warp waits for another
+// before the epilogue.
+// What bounded the shared ring was the bulk copies: an SM finishes one every 83 clocks however short it is, so pieces of a
 // weight row of 2 KB just keep up with HBM, shorter ones do not, and rings that fit twice on an SM had no room for longer ones.
-// The warp multiplies the same columns of every unit, so its share of the activations is fetched once, straight into MMA
-// fragments (XC > 0: K = 256 XC), or, for a long K, a stage ahead (XC = 0: K a multiple of 2,048): nothing is staged and no
-// barrier comes between the kernel ahead and the first MMA.  Only the epilogue needs the 1/rms of a handed-over norm, so the
-// warps form it beside the first unit; the epilogue warp also asks for the residual before the sums are there.
-// Measured on B200, us of a layer's four products (qkv, output, gate/up, down) in a captured chain, 1, 8 and 16 rows, before (all
-// warps on one ring of bulk copies) and now: hidden 2,048 35.1, 37.3, 47.2 and 29.1, 31.1, 34.2 (18.6 of bytes); hidden
-// 3,072 51.1, 55.0, 73.9 and 42.1, 44.8, 48.9 (30.8).  Activations staged in shared memory took 1 to 1.9 us of every product
-// (8 rows; 3.3 at 16), the shared ring 0.44 us for 16 KB.
+// Nothing is staged and no barrier comes between the kernel ahead and the first MMA.  Only the epilogue needs the 1/rms of a
+// handed-over norm, so the warps form it beside the first unit.
+// XC > 0 (K = 256 XC): the warp multiplies the same columns of every unit, so its share of the activations is fetched once,
+// straight into MMA fragments.  XC = 0 (a long K): it does not fit the registers, so a stage brings its columns of the activations
+// behind those of the weights, as many stages ahead.  Fetched into registers three stages ahead of their use they came too late:
+// an L2 answer stands behind 100 KB of weights on their way to the SM.  28,672 x 8,192, 1, 8 and 16 rows: 101, 102 and 98 us so,
+// 76, 76 and 84 through the ring (bulk copies 76, 87 and 95; 72 of bytes); 3,072 x 8,192 16, 17 and 17, now 12, 12 and 14.
+// The loops would take any K of whole stages (512 k in units of 16 rows, 1,024 in units of 8); the launcher passes the measured ones.
+// Measured on B200, us of a layer's four products (qkv, output, gate/up, down) in a captured chain, 1, 8 and 16 rows, all on bulk
+// copies and all on rings of warps: hidden 2,048 and inner 8,192 36.6, 38.7, 48.7 and 27.3, 28.2, 31.2 (18.6 of bytes); hidden
+// 3,072 54.1, 57.8, 77.4 and 41.0, 43.0, 46.3 (30.7); hidden 4,096 and inner 14,336, 1 and 8 rows, 92.9, 97.0 and 77.8, 79.2 (66.6).
+// Over 864 products (K 1,024 to 14,336, 32 to 128,256 columns, 1 to 16 rows) back to back, each on both forms, the rings of warps
+// take 0.36 to 1.03 of the bulk copies' time, but for 3,072 x 8,192 at one row (12.0 and 11.3 us).
 constexpr int FLOW_THREADS = CONSUMER_THREADS + 32;        // + the epilogue warp
 template <int NT>
-struct FlowShape {                                         // a stage: 16 KB over the block
+struct FlowShape {                                         // a stage: 16 KB of weights over the block
   static constexpr int CHUNKS = 4 / NT;                    // of 32 k, a warp
   static constexpr int K = 32 * CHUNKS, KS = K * CONSUMER_WARPS;
-  static constexpr int ROW_BYTES = 2 * K, STAGE_BYTES = 8 * NT * ROW_BYTES;
-  static constexpr int AHEAD = NT == 1 ? 2 : 4;            // buffers of activations of a long K
+  static constexpr int ROW_BYTES = 2 * K, W_BYTES = 8 * NT * ROW_BYTES;
 };
+// XC: chunks of 32 k a warp whose activations stay in registers (K = 256 XC); 0: activations through the ring
+template <int NT, bool TWO, int XC>
+constexpr int FLOW_SLOT_BYTES = FlowShape<NT>::W_BYTES + (XC > 0 ? 0 : (TWO ? 16 : 8) * FlowShape<NT>::ROW_BYTES);
 
 __device__ __forceinline__ void flow_copy16(uint32_t dst, const void* src, bool there, uint64_t pol) {
-  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0), "l"(pol) : "memory");
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;"
+               ::"r"(dst), "l"(src), "r"(there ? 16 : 0), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void flow_copy16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void flow_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -584,12 +599,12 @@ template <int NT, bool TWO, int XC, int STAGES>
 __device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* smem, float* red_mem, float* inv_rms) {
   using F = FlowShape<NT>;
   constexpr int UNIT_ROWS = 8 * NT, CHUNKS = F::CHUNKS, LANES = F::ROW_BYTES / 16, ROWS = 32 / LANES;
-  constexpr int XN = XC > 0 ? XC : F::AHEAD * CHUNKS;
+  constexpr int X_ROWS = TWO ? 16 : 8, SLOT_BYTES = FLOW_SLOT_BYTES<NT, TWO, XC>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n_units = (p.N + UNIT_ROWS - 1) / UNIT_ROWS;
   const int k_stages = XC > 0 ? XC / CHUNKS : p.K / F::KS;
   float (*red)[CONSUMER_WARPS][4 * NT][32] = reinterpret_cast<float (*)[CONSUMER_WARPS][4 * NT][32]>(red_mem);
-  const uint32_t ring = smem_addr(smem) + warp * (STAGES * F::STAGE_BYTES);
+  const uint32_t ring = smem_addr(smem) + warp * (STAGES * SLOT_BYTES);
 
   // ---- weights: 16-byte pieces of odd rows change halves of 128 bytes, so that the fragments' reads (8 rows, 4 pieces) touch
   // every bank once a quarter warp
@@ -599,11 +614,11 @@ __device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* 
   const int my_units = (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int total = my_units * k_stages;
   int unit = blockIdx.x, ksi = 0, issued = 0, slot_in = 0;
-  auto copy = [&]() {
+  auto copy_weights = [&]() {
     if (issued < total) {
       const int n0 = unit * UNIT_ROWS + cr;
       const bf16* src = p.W + (size_t)n0 * p.ldw + ksi * F::KS + warp * F::K + cc * 8;
-      const uint32_t dst = c_dst + slot_in * F::STAGE_BYTES;
+      const uint32_t dst = c_dst + slot_in * SLOT_BYTES;
 #pragma unroll
       for (int i = 0; i < UNIT_ROWS / ROWS; ++i) {
         const bool there = n0 + ROWS * i < p.N;
@@ -611,27 +626,57 @@ __device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* 
       }
       if (++ksi == k_stages) { ksi = 0; unit += gridDim.x; }
     }
-    flow_commit();
     ++issued;
     if (++slot_in == STAGES) slot_in = 0;
   };
 #pragma unroll
-  for (int s = 0; s < STAGES; ++s) copy();
+  for (int s = 0; s < STAGES; ++s) {
+    copy_weights();
+    flow_commit();
+  }
 
   // ---- activations, and the 1/rms of rows warp and warp + 8
-  const bf16* const xa = (const bf16*)p.A + (size_t)(g < p.M ? g : 0) * p.lda + warp * F::K + t * 8;
-  const bf16* const xb = (const bf16*)p.A + (size_t)(g + 8 < p.M ? g + 8 : 0) * p.lda + warp * F::K + t * 8;
-  const bool va = g < p.M, vb = g + 8 < p.M;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  uint4 x0[XN], x1[TWO ? XN : 1];
-  auto fetch = [&](int to, int offset) {
-    x0[to] = va ? __ldcg(reinterpret_cast<const uint4*>(xa + offset)) : zero;
-    if (TWO) x1[to] = vb ? __ldcg(reinterpret_cast<const uint4*>(xb + offset)) : zero;
-  };
-  pdl_wait();
-  constexpr int FIRST = XC > 0 ? XC : (F::AHEAD - 1) * CHUNKS;
+  // a long K: the same columns of the activations behind the weights of every stage (the rows beyond M are zeroed once)
+  const bf16* const x_src = (const bf16*)p.A + (size_t)cr * p.lda + warp * F::K + cc * 8;
+  int x_ksi = 0, x_issued = 0, x_slot_in = 0;
+  auto copy_activations = [&]() {
+    if (x_issued < total) {
+      const uint32_t dst = c_dst + F::W_BYTES + x_slot_in * SLOT_BYTES;
 #pragma unroll
-  for (int c = 0; c < FIRST; ++c) fetch(c, c / CHUNKS * F::KS + c % CHUNKS * 32);
+      for (int i = 0; i < X_ROWS / ROWS; ++i)
+        if (cr + ROWS * i < p.M) flow_copy16(dst + i * 512, x_src + (size_t)(ROWS * i) * p.lda + x_ksi * F::KS);
+      if (++x_ksi == k_stages) x_ksi = 0;
+    }
+    ++x_issued;
+    if (++x_slot_in == STAGES) x_slot_in = 0;
+  };
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  if (XC == 0) {
+#pragma unroll 1
+    for (int s = 0; s < STAGES; ++s)
+#pragma unroll
+      for (int i = 0; i < X_ROWS / ROWS; ++i)
+        if (cr + ROWS * i >= p.M) sts128(c_dst + F::W_BYTES + s * SLOT_BYTES + i * 512, zero);
+  }
+  uint4 x0[XC > 0 ? XC : 1], x1[XC > 0 && TWO ? XC : 1];
+  pdl_wait();
+  if (XC > 0) {
+    const bf16* const xa = (const bf16*)p.A + (size_t)(g < p.M ? g : 0) * p.lda + warp * F::K + t * 8;
+    const bf16* const xb = (const bf16*)p.A + (size_t)(g + 8 < p.M ? g + 8 : 0) * p.lda + warp * F::K + t * 8;
+    const bool va = g < p.M, vb = g + 8 < p.M;
+#pragma unroll
+    for (int c = 0; c < XC; ++c) {
+      const int offset = c / CHUNKS * F::KS + c % CHUNKS * 32;
+      x0[c] = va ? __ldcg(reinterpret_cast<const uint4*>(xa + offset)) : zero;
+      if (TWO) x1[c] = vb ? __ldcg(reinterpret_cast<const uint4*>(xb + offset)) : zero;
+    }
+  } else {
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) {
+      copy_activations();
+      flow_commit();
+    }
+  }
   float part[TWO ? 2 : 1];
   if (p.pro == PRO_PRENORMED) {
 #pragma unroll
@@ -639,7 +684,8 @@ __device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* 
       float v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        v[j] = warp + 8 * h < p.M && j * 32 + lane < p.ssq_blocks ? __ldcg(p.ssq_in + (size_t)(warp + 8 * h) * p.ssq_blocks + j * 32 + lane) : 0.f;
+        v[j] = warp + 8 * h < p.M && j * 32 + lane < p.ssq_blocks
+                   ? __ldcg(p.ssq_in + (size_t)(warp + 8 * h) * p.ssq_blocks + j * 32 + lane) : 0.f;
       part[h] = v[0];
 #pragma unroll
       for (int j = 1; j < 8; ++j) part[h] += v[j];
@@ -656,41 +702,36 @@ __device__ __forceinline__ void consume_flow(const TmaParams& p, unsigned char* 
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[nt][0][e] = acc[nt][1][e] = 0.f;
     auto stage = [&](int x_at) {
-      flow_wait<STAGES - 1>();
+      flow_wait<STAGES - 1>();                               // of the stages' last groups: weights, or activations behind them
       __syncwarp();
-      const uint32_t wbase = w_at + slot * F::STAGE_BYTES;
-      uint4 w[CHUNKS][NT];
+      const uint32_t wbase = w_at + slot * SLOT_BYTES;
+      uint4 w[CHUNKS][NT], a[CHUNKS], h[CHUNKS];
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c) {
+        const uint32_t piece = ((c * 4 + t) ^ odd) << 4;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) w[c][nt] = lds128(wbase + nt * 8 * F::ROW_BYTES + piece);
+        a[c] = XC > 0 ? x0[XC > 0 ? x_at + c : 0] : lds128(wbase + F::W_BYTES + piece);
+        h[c] = !TWO ? zero : XC > 0 ? x1[XC > 0 && TWO ? x_at + c : 0] : lds128(wbase + F::W_BYTES + 8 * F::ROW_BYTES + piece);
+      }
 #pragma unroll
       for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) w[c][nt] = lds128(wbase + nt * 8 * F::ROW_BYTES + (((c * 4 + t) ^ odd) << 4));
-#pragma unroll
-      for (int c = 0; c < CHUNKS; ++c) {
-        const uint4 a = x0[x_at + c], h = TWO ? x1[x_at + c] : zero;
-#pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-          mma16816(acc[nt][0], a.x, h.x, a.y, h.y, w[c][nt].x, w[c][nt].y);
-          mma16816(acc[nt][1], a.z, h.z, a.w, h.w, w[c][nt].z, w[c][nt].w);
+          mma16816(acc[nt][0], a[c].x, h[c].x, a[c].y, h[c].y, w[c][nt].x, w[c][nt].y);
+          mma16816(acc[nt][1], a[c].z, h[c].z, a[c].w, h[c].w, w[c][nt].z, w[c][nt].w);
         }
-      }
       __syncwarp();                                          // every lane has read the slot
-      copy();
+      copy_weights();
+      if (XC == 0) copy_activations();
+      flow_commit();
       if (++slot == STAGES) slot = 0;
     };
     if (XC > 0) {
 #pragma unroll
       for (int i = 0; i < (XC > 0 ? XC / CHUNKS : 1); ++i) stage(i * CHUNKS);
     } else {
-      for (int i = 0; i < k_stages; i += F::AHEAD) {
-#pragma unroll
-        for (int j = 0; j < F::AHEAD; ++j) {
-          // the columns of AHEAD - 1 stages on (of the next unit, if this one ends: they are the same)
-          const int next = i + j + F::AHEAD - 1 < k_stages ? i + j + F::AHEAD - 1 : i + j + F::AHEAD - 1 - k_stages;
-#pragma unroll
-          for (int c = 0; c < CHUNKS; ++c) fetch((j + F::AHEAD - 1) % F::AHEAD * CHUNKS + c, next * F::KS + c * 32);
-          stage(j * CHUNKS);
-        }
-      }
+      for (int i = 0; i < k_stages; ++i) stage(0);
     }
     if (n_done == 0 && p.pro == PRO_PRENORMED) {             // the epilogue warp reads them behind its first barrier
 #pragma unroll
@@ -962,7 +1003,9 @@ __global__ void __launch_bounds__(THREADS, 1) moe_ring_kernel(GroupedParams p) {
 template <int NT, int EPI>
 int launch_ring(const GroupedParams& p, int n_sms, size_t smem, cudaStream_t stream) {
   static OncePerDevice once;
-  const int ready = once([] { return cudaFuncSetAttribute(moe_ring_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024); });
+  const int ready = once([] {
+    return cudaFuncSetAttribute(moe_ring_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024);
+  });
   if (ready) return ready;
   return launch_k(moe_ring_kernel<NT, EPI>, n_sms, THREADS, smem, stream, p);
 }
@@ -970,10 +1013,14 @@ int launch_ring(const GroupedParams& p, int n_sms, size_t smem, cudaStream_t str
 // Products in rings of warps
 template <int NT, bool TWO, int XC>
 int launch_flow_as(const TmaParams& p, int n_sms, cudaStream_t stream) {
-  // Rings of 96 KB, 128 KB for a long K (44.8 us a layer of hidden 3,072 against 45.2; 64 KB: 46.3), and more shared memory than
-  // two blocks of an SM can have.  Blocks of the kernel behind would else take the places that blocks of this one leave early, two on one SM
-  // while others have none, and the slowest SM decides: 38.7 us with 90 KB a block where 120 KB take 31.1.
-  constexpr int STAGES = XC == 0 ? 8 : 6, smem = STAGES == 6 ? 120 * 1024 : STAGES * 16 * 1024;
+  // Rings of 96 KB where the activations stay in registers, and more shared memory than two blocks of an SM can have.  Blocks of
+  // the kernel behind would else take the places that blocks of this one leave early, two on one SM while others have none, and the
+  // slowest SM decides: 38.7 us a layer with 90 KB a block where 120 KB take 31.1.
+  // With activations in the ring 160 to 192 KB.  Fewer stages cost 3,072 x 4,096 9 to 12 % at 8 rows (6 or 7 instead of 8) and up to
+  // 5 % at 9 (3 instead of 4, units of 8 rows); 5 instead of 6 at 16 rows, units of 16, are as fast or up to 3 % faster a layer.
+  constexpr int STAGES = XC > 0 ? 6 : NT == 1 ? (TWO ? 4 : 6) : (TWO ? 5 : 8);
+  constexpr int smem = XC > 0 ? 120 * 1024 : STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC>;
+  static_assert(smem >= STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC> && smem > 114 * 1024, "the ring, and one block an SM");
   static OncePerDevice once;
   const int ready = once([] {
     return (int)cudaFuncSetAttribute(gemm_stream_flow_kernel<NT, TWO, XC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1086,7 +1133,11 @@ extern "C" int ie_gemm_stream_tma(const void* A, const void* W, void* C, const v
   if (pro == PRO_PRENORMED && (!ssq || ssq_blocks <= 0 || ssq_blocks > 256)) return IE_BAD_SIZE;
   p.pro = pro; p.epi = epi;
   if (pro != PRO_NORM && (K == 1024 || K == 2048 || K == 3072 || K % 2048 == 0)) {
-    // as below: units of 16 rows where every SM still gets several, or, for a long K, about one
+    // Units of 16 rows where every SM still gets several, or, for a long K, about one.  Up to 3,072 k the two are within 4 % for
+    // stores (us, units of 8 and of 16, 8 rows: 9,472 x 2,048 7.3 and 7.5, 32,768 x 2,048 22.1 and 22.1, 16,384 x 3,072 17.0 and
+    // 17.3), with half the epilogues for 1,024 k (32,768 of silu(gate) up 13.3 and 12.3).  A long K reads its activations half as
+    // often: 2,048 x 8,192 7.5 and 7.6 at 8 rows, 9.0 and 8.1 at 16; 16,384 x 4,096 26.2 and 23.0; but 512 x 8,192, where half the
+    // SMs would have none, 3.6 and 5.7.  (1,536 x 8,192, below the line, would take 7.3 and 6.5; 3,072 x 8,192, above it, 10.4 and 12.0.)
     const bool wide = N >= 16 * 4 * n_sms || (K > 3072 && (N + 15) / 16 >= (n_sms * 3) / 4);
     if (M > 8) return wide ? launch_flow<2, true>(p, n_sms, stream) : launch_flow<1, true>(p, n_sms, stream);
     return wide ? launch_flow<2, false>(p, n_sms, stream) : launch_flow<1, false>(p, n_sms, stream);

@@ -1,31 +1,41 @@
 // Persistent weight-streaming product for decode steps on sm_100a:
-// C[M,N] = A[M,K] W[N,K]^T, M <= 16, bfloat16 weights read once from HBM by the
-// bulk-copy engine (cp.async.bulk, completion on mbarriers) into a ring of shared
-// memory stages, one block per SM that walks units of 8 weight rows.
+// C[M,N] = A[M,K] W[N,K]^T, M <= 16, bfloat16 weights read once from HBM through rings of
+// shared memory stages, one block per SM that walks units of 8 or 16 weight rows.
 //
 // Why this shape: at M <= 16 the product is a read of W.  A block that owns little
 // data spends its life on latency (first bytes from HBM, activations from L2,
-// reduction, store); here a producer thread keeps the ring full across unit
-// boundaries, so HBM requests never stop while consumer warps multiply, reduce and
-// store.  Launched with programmatic dependent launch, the producer starts filling
-// the ring with this kernel's weights while the kernel ahead is still running; only
-// the consumers wait for its output.
+// reduction, store); here the rings are kept full across unit
+// boundaries, so HBM requests never stop while the warps multiply, reduce and
+// store.  Launched with programmatic dependent launch, a block starts filling
+// its rings with this kernel's weights while the kernel ahead is still running; only
+// the activations wait for its output.
 //
+// Two forms, chosen by the prologue and K (ie_gemm_stream_tma):
+//
+// rings of warps (gemm_stream_flow_kernel; bfloat16 activations, plain or handed over, K of 1,024, 2,048, 3,072 or a multiple
+// of 2,048: the widths of the models that were measured):
+//   warps 0-7: each streams an eighth of every stage's k through a ring of its own (cp.async, 16 bytes a lane), keeps its share
+//             of the activations in MMA fragments or brings it through the ring, and runs mma.sync m16n8k16
+//   warp 8:   the epilogue, as below
+//
+// bulk copies (gemm_stream_tma_kernel; a norm in the prologue, and every other K that is a multiple of 256):
 //   producer  warp 8: for every (unit, k-stage) wait for the stage to be
-//             free, arm its mbarrier with the byte count, issue one bulk copy per
+//             free, arm its mbarrier with the byte count, issue one bulk copy (cp.async.bulk) per
 //             weight row (rows are contiguous in global memory)
 //   consumers warps 0-7: stage the activations once per block in shared memory
 //             (bfloat16; with the RMSNorm prologue x*gain and 1/rms are computed here
-//             in float32, engine/layers.py:24-25), then per stage each warp takes a
-//             eighth of k, builds MMA fragments with 16-byte shared loads and runs
-//             mma.sync m16n8k16; at the end of a unit each warp leaves its partial sums in
-//             shared memory and goes on with the next unit
-//   epilogue  warp 9: adds the eight partial sums of a unit in warp order and applies the
-//             epilogue of gemm_stream.cu, one unit behind the consumers (two buffers of sums,
-//             handed over through named barriers)
+//             in float32, engine/layers.py:24-25) or, where they do not fit beside the ring, read them from L2, then per
+//             stage each warp takes an eighth of k, builds MMA fragments with 16-byte shared loads and runs
+//             mma.sync m16n8k16
+//   epilogue  warp 9
+//
+// In both, at the end of a unit each warp leaves its partial sums in shared memory and goes on with the next unit; the epilogue
+// warp adds the eight partial sums of a unit in warp order and applies the epilogue of gemm_stream.cu, one unit behind (two
+// buffers of sums, handed over through named barriers).
 //
 // Every wait on an mbarrier is bounded; on a timeout the block records an error
-// word that ie_gemm_stream_tma_error() reads, stops issuing copies and leaves.
+// word that ie_gemm_stream_tma_error() reads, stops issuing copies and leaves.  (The rings of warps wait for their own warp's
+// copies alone.)
 #include "common.cuh"
 
 namespace {
@@ -59,8 +69,8 @@ constexpr unsigned SPIN_LIMIT = IE_STREAM_SPIN_LIMIT;
 
 __device__ int g_stream_error = 0;
 
-// Diagnostics, compiled in with -DIE_STREAM_TRACE only: thread 0 of block 0 of every launch notes the GPU's
-// nanosecond clock at eight points of its life; ie_gemm_stream_trace_read() hands the notes to the host.
+// Diagnostics, compiled in with -DIE_STREAM_TRACE only: thread 0 of block 0 of every launch of the bulk copies' form notes the
+// GPU's nanosecond clock at eight points of its life; ie_gemm_stream_trace_read() hands the notes to the host.
 #ifdef IE_STREAM_TRACE
 constexpr int TRACE_LAUNCHES = 4096, TRACE_POINTS = 8;
 __device__ unsigned long long g_trace[TRACE_LAUNCHES * TRACE_POINTS];
@@ -80,7 +90,7 @@ __device__ __forceinline__ unsigned long long trace_now() {
 #endif
 
 struct TmaParams {
-  const void* A;          // PLAIN: bf16 [M, lda];  NORM: float32 residual rows [*, lda]
+  const void* A;          // PLAIN, PRENORMED: bf16 [M, lda];  NORM: float32 residual rows [*, lda]
   const bf16* W;          // [N, ldw]
   void* C;
   const void* gain;
@@ -88,7 +98,7 @@ struct TmaParams {
   int M, N, K, lda, ldw, ldc;
   int gain_is_f32;
   float eps;
-  int ks;                 // k elements per stage (multiple of 128)
+  int ks;                 // k elements per stage (multiple of 128); this and the three below: bulk copies
   int n_stages;
   int x_rows;             // 8 or 16 activation rows (one MMA tile of tokens)
   int x_in_smem;          // activations staged in shared memory once per block (else read from L2 per chunk)
@@ -101,7 +111,7 @@ struct TmaParams {
   const float* ssq_in;    // [SSQ_SLOT rows][ssq_blocks] the sums of the product ahead (PRENORMED)
   int ssq_blocks;
   float act_alpha, act_limit, act_offset, act_cubic;   // GLU
-  int pro, epi;           // products with activations in registers (their epilogue warp chooses as it runs)
+  int pro, epi;           // what the launcher was asked for (the epilogue scales by it; the rings of warps choose theirs by epi)
 };
 
 // the gated activation of the GLU epilogue: g' sigmoid(alpha g' + cubic g'^3) (u' + offset), g' = min(g, limit) and u' = u
@@ -349,7 +359,6 @@ __device__ __forceinline__ void consume(const TmaParams& p, const BlockCtx& b, R
   int parity = 0, n_done = 0;
   bool dead = false;   // after a timed-out wait a warp stops waiting and computing but still meets every barrier
   for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-    // two accumulators per n-tile: the two MMAs of a chunk do not wait for each other
     // two accumulators per n-tile: the two MMAs of a chunk do not wait for each other (4 and 8 per n-tile were
     // measured too: a step of 16 layers at batch 8 took 0.968 and 0.985 ms against 0.941, for the registers they cost)
     float acc[NT][ASETS][4];
@@ -780,8 +789,8 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) gemm_stream_flow_kernel(TmaPa
 
 // One product per launch.
 template <int NT, int PRO, int EPI, bool XS>
-// Units of 8 rows (short products: qkv, output) keep within 112 registers, so that the kernel behind them in
-// the stream (decode attention, say) finds room on the SM and starts its own fetches early.
+// Units of 8 rows (short products) keep within 112 registers, so that the kernel behind them in the stream (decode attention,
+// say) finds room on the SM and starts its own fetches early.
 __global__ void __launch_bounds__(THREADS, NT == 1 ? 2 : 1) gemm_stream_tma_kernel(TmaParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long bars[2 * MAX_STAGES];   // full[], empty[]
@@ -1064,10 +1073,12 @@ int launch_tma(const TmaParams& p, int nt, int n_sms, size_t smem, cudaStream_t 
 
 }  // namespace
 
-// 1 if the kernel takes this product (M <= 16, K a multiple of 256, activations fit in shared memory)
-// Activations are kept in shared memory when they take at most this much; beyond it the plain prologue
-// reads them from L2 and the RMSNorm prologue is not offered.
+// The bulk copies' form keeps activations in shared memory when they take at most this much; beyond it the plain prologue
+// reads them from L2 and a norm, in the prologue or handed over, is not offered.  (The rings of warps stage nothing and could take
+// handed-over rows of any length; callers choose the library product there, and nothing beyond the limit was measured.)
 constexpr size_t X_SMEM_LIMIT = 100 * 1024;
+
+// 1 if one of the two forms takes this product: M <= 16, K a multiple of 256, with a norm the rows within X_SMEM_LIMIT
 
 extern "C" int ie_gemm_stream_tma_supports(int M, int N, int K, int pro) {
   if (M <= 0 || M > 16 || N <= 0 || K <= 0 || (K % 256)) return 0;

@@ -641,8 +641,9 @@ __device__ __forceinline__ void cp_async_wait_pending(int pending) {
   }
 }
 
-// head size 64: at most 112 registers at 192 threads, so that the block fits beside the product kernels ahead of
-// and behind it in the stream
+// head size 64: at most 112 registers at 192 threads and 102 KB of shared memory, so that the block fits beside one of the product
+// kernels ahead of and behind it in the stream (gemm_stream_tma.cu: 117 to 125 KB; its registers leave room too, but for 9 to 16
+// rows of 3,072 columns)
 __global__ void __launch_bounds__(DC_THREADS, (HD <= 64 && !BIASED) ? 3 : 2) attention_decode_kernel(MmaAttnParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   pdl_trigger();

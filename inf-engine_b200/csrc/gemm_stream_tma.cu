@@ -1024,12 +1024,14 @@ template <int NT, bool TWO, int XC>
 int launch_flow_as(const TmaParams& p, int n_sms, cudaStream_t stream) {
   // Rings of 96 KB where the activations stay in registers, and more shared memory than two blocks of an SM can have.  Blocks of
   // the kernel behind would else take the places that blocks of this one leave early, two on one SM while others have none, and the
-  // slowest SM decides: 38.7 us a layer with 90 KB a block where 120 KB take 31.1.
+  // slowest SM decides: 38.7 us a layer with 90 KB a block where 120 KB take 31.1.  But no more than leaves room for a block of the
+  // decode attention for heads of 64 (102 KB), which asks for its first keys beside the product ahead: with 120 KB a decode step of
+  // the 1B size takes 623 us for one request and 751 for eight, with 108 KB 614 and 742.
   // With activations in the ring 160 to 192 KB.  Fewer stages cost 3,072 x 4,096 9 to 12 % at 8 rows (6 or 7 instead of 8) and up to
   // 5 % at 9 (3 instead of 4, units of 8 rows); 5 instead of 6 at 16 rows, units of 16, are as fast or up to 3 % faster a layer.
   constexpr int STAGES = XC > 0 ? 6 : NT == 1 ? (TWO ? 4 : 6) : (TWO ? 5 : 8);
-  constexpr int smem = XC > 0 ? 120 * 1024 : STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC>;
-  static_assert(smem >= STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC> && smem > 114 * 1024, "the ring, and one block an SM");
+  constexpr int smem = XC > 0 ? 108 * 1024 : STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC>;
+  static_assert(smem >= STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC> && 2 * (smem + 9 * 1024) > 228 * 1024, "the ring, and one block an SM");
   static OncePerDevice once;
   const int ready = once([] {
     return (int)cudaFuncSetAttribute(gemm_stream_flow_kernel<NT, TWO, XC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

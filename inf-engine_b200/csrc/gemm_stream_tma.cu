@@ -1031,7 +1031,8 @@ int launch_flow_as(const TmaParams& p, int n_sms, cudaStream_t stream) {
   // 5 % at 9 (3 instead of 4, units of 8 rows); 5 instead of 6 at 16 rows, units of 16, are as fast or up to 3 % faster a layer.
   constexpr int STAGES = XC > 0 ? 6 : NT == 1 ? (TWO ? 4 : 6) : (TWO ? 5 : 8);
   constexpr int smem = XC > 0 ? 108 * 1024 : STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC>;
-  static_assert(smem >= STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC> && 2 * (smem + 9 * 1024) > 228 * 1024, "the ring, and one block an SM");
+  static_assert(smem >= STAGES * CONSUMER_WARPS * FLOW_SLOT_BYTES<NT, TWO, XC>, "the rings fit");
+  static_assert(2 * (smem + 9 * 1024) > 228 * 1024, "one block an SM");
   static OncePerDevice once;
   const int ready = once([] {
     return (int)cudaFuncSetAttribute(gemm_stream_flow_kernel<NT, TWO, XC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
